@@ -23,6 +23,7 @@
 #include "assemble_mma.cuh"
 #include "assemble_p1.cuh"
 #include "cm_integrate.cuh"
+#include "cp_crystal.cuh"
 #include "cp_kernels.cuh"
 #include "neumann.cuh"
 #include "transient.cuh"
@@ -72,6 +73,8 @@ struct pgfem_gpu_ctx {
   int *cp_iters = nullptr;
   unsigned *cp_counter = nullptr;
   uint8_t *cp_conv = nullptr;  // per point: converged (the tangent kernel's input)
+  bool cp_rot = false;         // every crystal rotation is orthogonal: crystal-frame kernels
+  double *cp_rec = nullptr;    // element records of the crystal-frame element stage
   bool cp_use_guess = false;
   // learned warm start: F at t_n, network features / predictions, cold restarts
   double *cp_Fn = nullptr;
@@ -336,7 +339,7 @@ void release(pgfem_gpu_ctx *c) {
                   c->cp_R, c->cp_F, c->cp_detJw, c->cp_out, c->cp_guess, c->cp_iters, c->cp_counter,
                   c->cp_Fn, c->cp_feat, c->cp_pred, c->cp_fallbacks, c->elem_group, c->F0_tab, c->cp_conv,
                   c->sched_ticket, c->p2m_ticket, c->tf_P, c->tf_theta, c->tf_dunode, c->tf_inc, c->nbc_desc_tr, c->nbc_elem, c->nbc_feat, c->nbc_type, c->nbc_off, c->nbc_face,
-                  c->nbc_load, c->tr_buf, c->state_nm1, c->tr_F, c->tf_hist, c->tf_mid, c->mass_csr};
+                  c->nbc_load, c->tr_buf, c->state_nm1, c->tr_F, c->tf_hist, c->tf_mid, c->mass_csr, c->cp_rec};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (c->zfork) cudaEventDestroy(c->zfork);
@@ -591,6 +594,41 @@ struct CpTransient {
   double alpha, cA, cB;
 };
 
+// The sample-frame local Newton (any crystal matrix): a persistent grid of the
+// resident CTAs.
+int launch_cp_update(const CpArgs &a, cudaStream_t s) {
+  const size_t smem = cp_update_smem();
+  static bool attr = false;
+  if (!attr) {
+    CK(cudaFuncSetAttribute(k_cp_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attr = true;
+  }
+  int per_sm = 0;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cp_update, 32 * kCpWarps, smem));
+  if (per_sm < 1) per_sm = 1;
+  if (!g_num_sms) grid_for(1, 1, 1);
+  const long need = (a.nqp + 32 * kCpWarps - 1) / (32 * kCpWarps);
+  const long grid = std::max<long>(1, std::min<long>(need, (long)g_num_sms * per_sm));
+  k_cp_update<<<(unsigned)grid, 32 * kCpWarps, smem, s>>>(a);
+  CK(cudaGetLastError());
+  return PGFEM_GPU_OK;
+}
+
+// The crystal-frame local Newton: a persistent grid of the resident CTAs, fewer
+// points a CTA (one warp's worth) when the batch does not fill it.
+int launch_cp_update_cx(const CpArgs &a, cudaStream_t s) {
+  auto kern = k_cp_update_cx<28>;
+  int per_sm = 0;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kCxWarps, 0));
+  if (per_sm < 1) per_sm = 1;
+  if (!g_num_sms) grid_for(1, 1, 1);
+  const long need = (a.nqp + 31) / 32;
+  const long grid = std::max<long>(1, std::min<long>(need, (long)g_num_sms * per_sm));
+  kern<<<(unsigned)grid, 32 * kCxWarps, 0, s>>>(a);
+  CK(cudaGetLastError());
+  return PGFEM_GPU_OK;
+}
+
 // The CP path: F per element, the local Newton (optionally from the network's
 // guess), the consistent tangent, then the element stage -- scattered into the
 // CSR (d_R, d_K) or, with el, the listed elements' dense blocks.
@@ -634,21 +672,36 @@ int assemble_cp(pgfem_gpu_ctx *c, double *d_R, double *d_K, double dt, cudaStrea
   a.status = c->status;
   a.mat = c->mat;
   a.dt = dt;
-  const size_t smem = cp_update_smem();
-  static bool attr = false;
-  if (!attr) {
-    CK(cudaFuncSetAttribute(k_cp_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr = true;
-  }
-  int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cp_update, 32 * kCpWarps, smem));
-  if (per_sm < 1) per_sm = 1;
-  if (!g_num_sms) grid_for(1, 1, 1);
-  const long need = (c->nqp + 32 * kCpWarps - 1) / (32 * kCpWarps);
-  const long grid = std::max<long>(1, std::min<long>(need, (long)g_num_sms * per_sm));
-  k_cp_update<<<(unsigned)grid, 32 * kCpWarps, smem, s>>>(a);
-  CK(cudaGetLastError());
-  {  // consistent tangent dM/dF of the converged points
+  const bool records = c->cp_rot && !el && !tr && d_R;  // element records instead of dM/dF
+  if (int r = c->cp_rot ? launch_cp_update_cx(a, s) : launch_cp_update(a, s)) return r;
+  CpElemArgs b{};
+  b.X = c->X;
+  b.conn = c->conn;
+  b.dof = c->dof;
+  b.rowptr0 = c->rowptr0;
+  b.rowlen = c->rowlen;
+  b.mask = c->mask;
+  b.pos = c->pos;
+  b.nn = c->nn;
+  b.ne = c->ne;
+  b.F = c->cp_F;
+  b.detJw = c->cp_detJw;
+  b.state_n = c->state_n;
+  b.out = c->cp_out;
+  b.R = d_R;
+  b.K = d_K;
+  b.mat = c->mat;
+  CxElemArgs x{};
+  x.e = b;
+  x.e.status = c->status;
+  x.Rcp = c->cp_R;
+  x.conv = c->cp_conv;
+  x.dt = dt;
+  x.rec = c->cp_rec;
+  if (records) {
+    k_cp_record_cx<<<(unsigned)((c->ne + 127) / 128), 128, 0, s>>>(x);
+    CK(cudaGetLastError());
+  } else {  // consistent tangent dM/dF of the converged points
     const size_t tsm = cp_tangent_smem();
     static bool tattr = false;
     if (!tattr) {
@@ -667,23 +720,6 @@ int assemble_cp(pgfem_gpu_ctx *c, double *d_R, double *d_K, double dt, cudaStrea
     c->events.emplace_back(e0, e1);
   }
   if (d_K || d_R || el) {
-    CpElemArgs b{};
-    b.X = c->X;
-    b.conn = c->conn;
-    b.dof = c->dof;
-    b.rowptr0 = c->rowptr0;
-    b.rowlen = c->rowlen;
-    b.mask = c->mask;
-    b.pos = c->pos;
-    b.nn = c->nn;
-    b.ne = c->ne;
-    b.F = c->cp_F;
-    b.detJw = c->cp_detJw;
-    b.state_n = c->state_n;
-    b.out = c->cp_out;
-    b.R = d_R;
-    b.K = d_K;
-    b.mat = c->mat;
     if (tr) {  // mid-point rule: R into d_R, K (if any) into d_K
       b.F_n = tr->F_n;
       b.F_nm1 = tr->F_nm1;
@@ -703,6 +739,11 @@ int assemble_cp(pgfem_gpu_ctx *c, double *d_R, double *d_K, double dt, cudaStrea
       b.lk_out = el->lk;
       b.fe_out = el->fe;
       k_cp_element<<<(unsigned)((el->n + 127) / 128), 128, 0, s>>>(b);
+      CK(cudaGetLastError());
+      return PGFEM_GPU_OK;
+    }
+    if (records) {
+      k_cp_scatter_cx<<<(unsigned)((c->ne + kCxTile - 1) / kCxTile), kCxElemThreads, 0, s>>>(x);
       CK(cudaGetLastError());
       return PGFEM_GPU_OK;
     }
@@ -791,7 +832,7 @@ int assemble_device(pgfem_gpu_ctx *c, const double *d_u, const double *d_presc, 
   }
   if (c->model == PGFEM_MODEL_CP) {
     int r;
-    if (!d_K) {  // residual only: the tangent columns are skipped by a scratch K
+    if (!d_K && !c->cp_rot) {  // residual only: the stiffness goes to a scratch K
       r = ensure_K_scratch(c);
       if (r) return r;
       CK(cudaMemsetAsync(c->d_K, 0, sizeof(double) * c->nnz, s));
@@ -840,6 +881,18 @@ int read_status(pgfem_gpu_ctx *c, pgfem_gpu_status *st, bool clear) {
   }
   if (clear) CK(cudaMemsetAsync(c->status, 0, sizeof(h), c->stream));
   return PGFEM_GPU_OK;
+}
+
+// Whether every crystal matrix is orthogonal to 1e-12 (R^T R = 1): the
+// crystal-frame kernels need it, others run the sample-frame ones.
+bool cp_rotations_orthogonal(const double *R, long ne) {
+  for (long e = 0; e < ne; e++, R += 9)
+    for (int i = 0; i < 3; i++)
+      for (int j = i; j < 3; j++) {
+        const double d = R[i] * R[j] + R[3 + i] * R[3 + j] + R[6 + i] * R[6 + j] - (i == j ? 1.0 : 0.0);
+        if (!(std::fabs(d) <= 1e-12)) return false;
+      }
+  return true;
 }
 
 // Greedy colouring: elements of one colour share no node, so their R and K
@@ -1085,12 +1138,14 @@ int pgfem_gpu_create(const pgfem_mesh_desc *m, const pgfem_material_desc *mat, c
   // crystal plasticity buffers (rotations SoA, F, point outputs)
   if (c->model == PGFEM_MODEL_CP) {
     std::vector<double> Rs((size_t)9 * ne);
+    c->cp_rot = cp_rotations_orthogonal(m->R_cp, ne);
     for (long e = 0; e < ne; e++)
       for (int i = 0; i < 9; i++) Rs[(size_t)i * ne + e] = m->R_cp[e * 9 + i];
     if ((r = upload(c, &c->cp_R, Rs.data(), Rs.size())) || (r = dalloc(c, &c->cp_F, (size_t)9 * ne)) ||
         (r = dalloc(c, &c->cp_detJw, ne)) || (r = dalloc(c, &c->cp_out, (size_t)kCpOut * c->nqp)) ||
         (r = dalloc(c, &c->cp_iters, c->nqp)) || (r = dalloc(c, &c->cp_counter, 1)) ||
-        (r = dalloc(c, &c->cp_fallbacks, 1)) || (r = dalloc(c, &c->cp_conv, c->nqp)))
+        (r = dalloc(c, &c->cp_fallbacks, 1)) || (r = dalloc(c, &c->cp_conv, c->nqp)) ||
+        (c->cp_rot && (r = dalloc(c, &c->cp_rec, (size_t)kCxRec * kCxTile * ((ne + kCxTile - 1) / kCxTile)))))
       return fail(r);
     std::vector<double> Fn((size_t)9 * c->nqp, 0.0);  // F at t_n: identity until the first commit
     for (long q = 0; q < c->nqp; q++) Fn[0 * c->nqp + q] = Fn[4 * c->nqp + q] = Fn[8 * c->nqp + q] = 1.0;
