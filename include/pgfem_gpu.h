@@ -382,10 +382,11 @@ int pgfem_gpu_cp_integrate_noalloc(const pgfem_material_desc *mat, long nqp, con
  * The CSR is block diagonal over the groups (one Psparse_ApAi pattern over
  * the union).  HE and J2. */
 int pgfem_gpu_set_mesh_groups(pgfem_gpu_ctx *ctx, int ngroups, const long *elem_off, const double *F0);
-/* Launch schedule of the linear-tet element kernel: elements per block
- * (16, 32, 64; 0 = default 32) and work stealing (grab > 0: a persistent
- * grid claims `grab` blocks of elements at a time from a counter; 0 = static
- * grid-stride order).  No counterpart in the reference. */
+/* Launch schedule of the linear-tet assembly: elements per block (16, 32, 64;
+ * 0 = default 32; where the owners of the rows assemble, 1, 2 or 4 warps per
+ * block) and work stealing (grab > 0: a persistent grid claims `grab` blocks of
+ * elements -- row owners -- at a time from a counter; 0 = static grid-stride
+ * order).  No counterpart in the reference. */
 int pgfem_gpu_set_schedule(pgfem_gpu_ctx *ctx, int elems_per_block, int grab);
 int pgfem_gpu_get_schedule(const pgfem_gpu_ctx *ctx, int *elems_per_block, int *grab);
 /* One R+K assembly on device buffers captured as a CUDA graph (the

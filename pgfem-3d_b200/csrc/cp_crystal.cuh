@@ -22,8 +22,9 @@
 // A point iteration takes about 1.3 k FP64 instructions and no shared-memory
 // matrix.  Measured at 663,552 points, load step 10 (48^3 cells): cold local
 // update 18.9 -> 1.19 ms, tangent 3.18 ms -> element records 0.22 ms, whole R+K
-// iterate 23.2 -> 1.88 ms, from a guess (3.6 iterations) 12.5 -> 1.36 ms; 7,986
-// points 1.00 -> 0.11 ms.  The update is bound by fixed-latency waits and the
+// iterate 23.2 -> 1.76 ms, from a guess (3.6 iterations) 12.5 -> 1.25 ms; 7,986
+// points 0.99 -> 0.10 ms (R and K by the row owners, assemble_gather.cuh; the
+// scatter below, for meshes without their lists, takes 0.1 ms more).  The update is bound by fixed-latency waits and the
 // FP64 pipe (54 % busy) at 8 warps per SM: 254 registers hold a point's state
 // and the reduced matrix; at 168 registers (12 warps) spills cost more than
 // the warps gain (2.03 ms an iterate).
@@ -550,19 +551,19 @@ __global__ void __launch_bounds__(32 * kCxWarps, 2) k_cp_update_cx(const CpArgs 
 // Element record: G = (dX/dxi)^-1 F^-1 (p_a = G^T dN_a/dxi), w tau (Voigt) and
 // the 36 numbers w c_(kl)(ij) of the spatial tangent, c : d = d tau - d tau -
 // tau d for symmetric d (columns kl of d, rows ij); zeros for an element without
-// contribution.  Tiles of 32 elements, field-major inside a tile: one thread per
-// element writes, and a scatter CTA reads its tile, in whole lines (element by
-// element instead: 312 against 222 us for the record kernel at 663,552 elements).
-constexpr int kCxRec = 51;
+// contribution.  Contiguous per element, padded to 16 bytes; turned in shared
+// memory so that a CTA writes its records in whole lines.
+constexpr int kCxRec = 52;
 constexpr int kCxT = 9, kCxC = 15;
-constexpr int kCxTile = 32;
+constexpr int kCxRecThreads = 64;
+constexpr int kCxTile = 32;  // elements per CTA of the scatter
 
 struct CxElemArgs {
   CpElemArgs e;
   const double *Rcp;
   const uint8_t *conv;
   double dt;
-  double *rec;  // kCxRec * ne, padded to whole tiles
+  double *rec;  // kCxRec * ne
 };
 
 // Kirchhoff stress tau = pJ (a dev(be) + kappa J (J - 1) 1), be = Fe Fe^T, and
@@ -576,12 +577,10 @@ struct CxElemArgs {
 // instead of 81: the update is objective, so only symmetric d count.  Points
 // that did not converge, or whose system is singular (counted in status[3]),
 // keep l = 0.
-__global__ void __launch_bounds__(128) k_cp_record_cx(const CxElemArgs B) {
+__device__ __forceinline__ void cx_record(const CxElemArgs &B, long e, double *rec) {
   const CpElemArgs &A = B.e;
-  const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (e >= A.ne) return;
   const long S = A.ne;
-  double *rec = B.rec + (e / kCxTile) * kCxTile * kCxRec + e % kCxTile;  // field f at f * kCxTile
+  rec[kCxRec - 1] = 0.0;
   const double w = A.detJw[e];
   double H[9], Mu[9], be[6], tau[6];
   double Gc[9], Mi[9], E6[6][6];  // E6: right-hand sides, then solutions
@@ -646,7 +645,7 @@ __global__ void __launch_bounds__(128) k_cp_record_cx(const CxElemArgs B) {
     }
   }
   if (!ok) {
-    for (int i = 0; i < kCxRec; i++) rec[i * kCxTile] = 0.0;
+    for (int i = 0; i < kCxRec; i++) rec[i] = 0.0;
     return;
   }
   const int vk[6] = {0, 1, 2, 1, 0, 0}, vl[6] = {0, 1, 2, 2, 2, 1};
@@ -702,11 +701,11 @@ __global__ void __launch_bounds__(128) k_cp_record_cx(const CxElemArgs B) {
       double z = a * ((v < 3 ? Sl[v] - s3 : Sl[v]) - (2.0 / 3.0) * (v < 3 ? be[q] : 0.0) - (2.0 / 3.0) * x * dev_be);
       if (v == q) z += dq * ((2.0 / 3.0) * a * trb - 2.0 * pv);
       if (v < 3) z += dpv * x;
-      rec[(kCxC + q * 6 + v) * kCxTile] = wp * (z - trl * tau[v]);
+      rec[kCxC + q * 6 + v] = wp * (z - trl * tau[v]);
     }
   }
 #pragma unroll
-  for (int v = 0; v < 6; v++) rec[(kCxT + v) * kCxTile] = wp * tau[v];
+  for (int v = 0; v < 6; v++) rec[kCxT + v] = wp * tau[v];
   // G = (dX/dxi)^-1 F^-1
   double x[4][3], dX[9], dXi[9], F[9], Fi[9], G[9];
 #pragma unroll
@@ -725,7 +724,17 @@ __global__ void __launch_bounds__(128) k_cp_record_cx(const CxElemArgs B) {
   inv3(F, Fi);
   mm3(dXi, Fi, G);
 #pragma unroll
-  for (int i = 0; i < 9; i++) rec[i * kCxTile] = G[i];
+  for (int i = 0; i < 9; i++) rec[i] = G[i];
+}
+
+__global__ void __launch_bounds__(kCxRecThreads) k_cp_record_cx(const CxElemArgs B) {
+  __shared__ double srow[kCxRecThreads * (kCxRec + 1)];
+  const long e0 = blockIdx.x * (long)kCxRecThreads, e = e0 + threadIdx.x;
+  if (e < B.e.ne) cx_record(B, e, srow + threadIdx.x * (kCxRec + 1));
+  __syncthreads();
+  const int cnt = (int)(B.e.ne - e0 < kCxRecThreads ? B.e.ne - e0 : kCxRecThreads) * kCxRec;
+  for (int i = threadIdx.x; i < cnt; i += kCxRecThreads)
+    B.rec[e0 * kCxRec + i] = srow[(i / kCxRec) * (kCxRec + 1) + i % kCxRec];
 }
 
 // R and K from the element records: K_ab[i][k] = p_a[j] c_(ij)(kl) p_b[l] +
@@ -735,16 +744,17 @@ __global__ void __launch_bounds__(128) k_cp_record_cx(const CxElemArgs B) {
 constexpr int kCxElemThreads = 12 * kCxTile;
 __global__ void __launch_bounds__(kCxElemThreads) k_cp_scatter_cx(const CxElemArgs B) {
   const CpElemArgs &A = B.e;
-  __shared__ double sm[kCxTile * kCxRec];
+  __shared__ double sm[kCxTile * (kCxRec + 1)];
   const long e0 = (long)blockIdx.x * kCxTile;
   const int tid = threadIdx.x;
   const int nel = (int)(A.ne - e0 < kCxTile ? A.ne - e0 : kCxTile);
-  for (int i = tid; i < kCxTile * kCxRec; i += kCxElemThreads) sm[i] = B.rec[e0 * kCxRec + i];
+  for (int i = tid; i < nel * kCxRec; i += kCxElemThreads)
+    sm[(i / kCxRec) * (kCxRec + 1) + i % kCxRec] = B.rec[e0 * kCxRec + i];
   __syncthreads();
   const int el = tid / 12, r = tid - el * 12, a = r / 3, k = r - a * 3;
   if (el >= nel) return;
   const long e = e0 + el;
-  auto rec = [&](int f) { return sm[f * kCxTile + el]; };
+  auto rec = [&](int f) { return sm[el * (kCxRec + 1) + f]; };
   const int na = A.conn[(long)a * A.ne + e];
   const unsigned ma = A.mask[na];
   if (!ma) return;

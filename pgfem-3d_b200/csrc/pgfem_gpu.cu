@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "assemble.cuh"
+#include "assemble_gather.cuh"
 #include "assemble_mma.cuh"
 #include "assemble_p1.cuh"
 #include "cm_integrate.cuh"
@@ -76,6 +77,12 @@ struct pgfem_gpu_ctx {
   bool cp_rot = false;         // every crystal rotation is orthogonal: crystal-frame kernels
   double *cp_rec = nullptr;    // element records of the crystal-frame element stage
   bool cp_use_guess = false;
+  // linear tets: lists of the row owners (gather assembly), HE / J2 records
+  bool gather = false;
+  GatherLists gl;
+  int g_per_sm[3] = {0, 0, 0};
+  void *g_mem[4] = {nullptr, nullptr, nullptr, nullptr};  // the lists' arrays
+  double *p1rec = nullptr;
   // learned warm start: F at t_n, network features / predictions, cold restarts
   double *cp_Fn = nullptr;
   float *cp_feat = nullptr, *cp_pred = nullptr;
@@ -339,8 +346,10 @@ void release(pgfem_gpu_ctx *c) {
                   c->cp_R, c->cp_F, c->cp_detJw, c->cp_out, c->cp_guess, c->cp_iters, c->cp_counter,
                   c->cp_Fn, c->cp_feat, c->cp_pred, c->cp_fallbacks, c->elem_group, c->F0_tab, c->cp_conv,
                   c->sched_ticket, c->p2m_ticket, c->tf_P, c->tf_theta, c->tf_dunode, c->tf_inc, c->nbc_desc_tr, c->nbc_elem, c->nbc_feat, c->nbc_type, c->nbc_off, c->nbc_face,
-                  c->nbc_load, c->tr_buf, c->state_nm1, c->tr_F, c->tf_hist, c->tf_mid, c->mass_csr, c->cp_rec};
+                  c->nbc_load, c->tr_buf, c->state_nm1, c->tr_F, c->tf_hist, c->tf_mid, c->mass_csr, c->cp_rec, c->p1rec};
   for (void *p : ptrs)
+    if (p) cudaFree(p);
+  for (void *p : c->g_mem)
     if (p) cudaFree(p);
   if (c->zfork) cudaEventDestroy(c->zfork);
   if (c->zjoin) cudaEventDestroy(c->zjoin);
@@ -530,6 +539,63 @@ int launch_p1r(pgfem_gpu_ctx *c, const AsmArgs &a, cudaStream_t s) {
   return launch_p1ws_te<MODEL, 16>(c, a, s);
 }
 
+// R and K of a linear-tet context from element records, by the owners of the
+// rows: the context's schedule gives the warps per CTA (elements per block 16, 32
+// or unset, 64: 1, 2, 4) and the groups claimed at a time.
+template <int MODEL>
+int launch_gather(pgfem_gpu_ctx *c, const double *rec, double *R, double *K, cudaStream_t s) {
+  const int sel = c->sched_epb == 16 ? 0 : (c->sched_epb == 64 ? 2 : 1), nw = 1 << sel;
+  const size_t smem = (size_t)nw * gather_plan(MODEL, c->gl.most, c->gl.slots, c->gl.packs, c->gl.width).bytes;
+  auto kern = k_gather_p1<MODEL>;
+  if (!c->g_per_sm[sel]) {
+    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGatherSmem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->g_per_sm[sel], kern, 32 * nw, smem));
+    if (c->g_per_sm[sel] < 1) c->g_per_sm[sel] = 1;
+  }
+  if (!g_num_sms) grid_for(1, 1, 1);
+  GatherArgs a{};
+  a.L = c->gl;
+  a.rec = rec;
+  a.R = R;
+  a.K = K;
+  if (c->sched_grab > 0) {
+    a.ticket = c->sched_ticket;
+    a.grab = c->sched_grab;
+    CK(cudaMemsetAsync(a.ticket, 0, sizeof(unsigned), s));
+  }
+  const long need = (c->gl.ng + nw - 1) / nw;
+  const long grid = std::max<long>(1, std::min<long>(need, (long)g_num_sms * c->g_per_sm[sel]));
+  kern<<<(unsigned)grid, 32 * nw, smem, s>>>(a);
+  CK(cudaGetLastError());
+  return PGFEM_GPU_OK;
+}
+
+// Linear tets, HE or J2: point update (displacements through the DOF ids) and
+// gather.
+template <int MODEL>
+int launch_p1_gather(pgfem_gpu_ctx *c, const double *d_u, const double *d_presc, double *R, double *K,
+                     cudaStream_t s) {
+  P1PointArgs q{};
+  q.X = c->X;
+  q.conn = c->conn;
+  q.dof = c->dof;
+  q.nn = c->nn;
+  q.ne = c->ne;
+  q.u = d_u;
+  q.presc = d_presc;
+  q.F0 = c->F0;
+  q.elem_group = c->elem_group;
+  q.F0_tab = c->F0_tab;
+  q.state_n = c->state_n;
+  q.state_np1 = c->state_np1;
+  q.rec = c->p1rec;
+  q.status = c->status;
+  q.mat = c->mat;
+  k_p1_points<MODEL><<<(unsigned)((c->ne + 127) / 128), 128, 0, s>>>(q);
+  CK(cudaGetLastError());
+  return launch_gather<MODEL>(c, c->p1rec, R, K, s);
+}
+
 template <bool ATOMIC, bool WANT_K, bool DENSE>
 int dispatch(pgfem_gpu_ctx *c, const AsmArgs &a, long nitems, cudaStream_t s) {
   // HE with the linear deviatoric potential: its tangent is carried by the
@@ -699,7 +765,7 @@ int assemble_cp(pgfem_gpu_ctx *c, double *d_R, double *d_K, double dt, cudaStrea
   x.dt = dt;
   x.rec = c->cp_rec;
   if (records) {
-    k_cp_record_cx<<<(unsigned)((c->ne + 127) / 128), 128, 0, s>>>(x);
+    k_cp_record_cx<<<(unsigned)((c->ne + kCxRecThreads - 1) / kCxRecThreads), kCxRecThreads, 0, s>>>(x);
     CK(cudaGetLastError());
   } else {  // consistent tangent dM/dF of the converged points
     const size_t tsm = cp_tangent_smem();
@@ -742,6 +808,7 @@ int assemble_cp(pgfem_gpu_ctx *c, double *d_R, double *d_K, double dt, cudaStrea
       CK(cudaGetLastError());
       return PGFEM_GPU_OK;
     }
+    if (records && c->gather) return launch_gather<2>(c, c->cp_rec, d_R, d_K, s);
     if (records) {
       k_cp_scatter_cx<<<(unsigned)((c->ne + kCxTile - 1) / kCxTile), kCxElemThreads, 0, s>>>(x);
       CK(cudaGetLastError());
@@ -812,6 +879,15 @@ bool uses_p2m(const pgfem_gpu_ctx *c) {
   return c->eblk && c->model != PGFEM_MODEL_CP && c->mat.dev_pot != 2 && c->scatter_mode == PGFEM_SCATTER_ATOMIC;
 }
 
+// Whether this call's R and K are written by the owners of the rows: linear tets
+// whose lists could be built, default scatter, R and K wanted (crystal plasticity:
+// R alone too).  The failure-path test of the hand-off waits runs the pipeline.
+bool gathers(const pgfem_gpu_ctx *c, const double *d_R, const double *d_K) {
+  if (!c->gather || !d_R) return false;
+  if (c->model == PGFEM_MODEL_CP) return c->cp_rot;
+  return d_K && c->scatter_mode == PGFEM_SCATTER_ATOMIC && !c->stall_next;
+}
+
 // One assembly on device buffers (zeroing R and K first).
 int assemble_device(pgfem_gpu_ctx *c, const double *d_u, const double *d_presc, double *d_R,
                     double *d_K, cudaStream_t s, double dt = 0.0) {
@@ -822,10 +898,11 @@ int assemble_device(pgfem_gpu_ctx *c, const double *d_u, const double *d_presc, 
       d_K = c->d_K;
     }
   }
-  if (d_R) CK(cudaMemsetAsync(d_R, 0, sizeof(double) * c->ndof, s));
+  const bool own = gathers(c, d_R, d_K);  // the row owners write every entry of R and K
+  if (d_R && !own) CK(cudaMemsetAsync(d_R, 0, sizeof(double) * c->ndof, s));
   // the tensor-core quadratic-tet path zeroes K itself, beside its point kernel
-  if (d_K && !(uses_p2m(c) && d_R)) CK(cudaMemsetAsync(d_K, 0, sizeof(double) * c->nnz, s));
-  {
+  if (d_K && !own && !(uses_p2m(c) && d_R)) CK(cudaMemsetAsync(d_K, 0, sizeof(double) * c->nnz, s));
+  if (!own || c->model == PGFEM_MODEL_CP || c->nbc_nface) {
     const long n3 = 3 * c->nn;
     k_expand_u<<<(unsigned)((n3 + 255) / 256), 256, 0, s>>>(c->dof, c->nn, d_u, d_presc, c->unode);
     CK(cudaGetLastError());
@@ -852,7 +929,10 @@ int assemble_device(pgfem_gpu_ctx *c, const double *d_u, const double *d_presc, 
     CK(cudaEventRecord(e0, s));
   }
   int r = PGFEM_GPU_OK;
-  if (c->scatter_mode == PGFEM_SCATTER_COLOUR && c->colour_elems) {
+  if (own) {
+    r = c->model == PGFEM_MODEL_J2 ? launch_p1_gather<1>(c, d_u, d_presc, d_R, d_K, s)
+                                   : launch_p1_gather<0>(c, d_u, d_presc, d_R, d_K, s);
+  } else if (c->scatter_mode == PGFEM_SCATTER_COLOUR && c->colour_elems) {
     for (size_t k = 0; k + 1 < c->colour_off.size() && !r; k++) {
       a.elist = c->colour_elems + c->colour_off[k];
       a.nlist = c->colour_off[k + 1] - c->colour_off[k];
@@ -895,18 +975,144 @@ bool cp_rotations_orthogonal(const double *R, long ne) {
   return true;
 }
 
+// Lists of the row owners of a linear-tet mesh (assemble_gather.cuh).  A group is
+// the nodes with the same free DOFs; leaves c->gather false when DOFs are shared
+// in any other way, when a DOF belongs to no node, when a row holds columns that
+// no element couples, or when a group has more incidences than the lists allow.
+int build_gather(pgfem_gpu_ctx *c, const std::vector<int> &dof, const std::vector<int> &rowptr0,
+                 const std::vector<int> &rowlen, const std::vector<uint8_t> &mask) {
+  const long nn = c->nn, ne = c->ne;
+  std::vector<int> rep((size_t)c->ndof, -1), owner((size_t)c->ndof, -1), grp((size_t)nn, -1);
+  for (long n = 0; n < nn; n++) {
+    if (!mask[n]) continue;
+    int first = -1;
+    for (int i = 0; i < 3; i++) {
+      const int id = dof[(size_t)i * nn + n];
+      if (id <= 0) continue;
+      if (first < 0) first = id - 1;
+      if (owner[id - 1] >= 0 && owner[id - 1] != first) return PGFEM_GPU_OK;
+      owner[id - 1] = first;
+    }
+    if (rep[first] < 0) rep[first] = (int)n;
+    const long m = rep[first];
+    for (int i = 0; i < 3; i++)
+      if (dof[(size_t)i * nn + n] > 0 ? dof[(size_t)i * nn + n] != dof[(size_t)i * nn + m]
+                                      : dof[(size_t)i * nn + m] > 0)
+        return PGFEM_GPU_OK;
+  }
+  std::vector<int4> row;
+  std::vector<int> gid((size_t)c->ndof, -1);
+  for (long d = 0; d < c->ndof; d++) {
+    if (owner[d] < 0) return PGFEM_GPU_OK;
+    if (rep[d] < 0) continue;
+    gid[d] = (int)row.size();
+    row.push_back(make_int4(rowptr0[rep[d]], rowlen[rep[d]], (int)d, mask[rep[d]]));
+  }
+  const long ng = (long)row.size();
+  if (!ng) return PGFEM_GPU_OK;
+  for (long n = 0; n < nn; n++)
+    for (int i = 2; mask[n] && i >= 0; i--)
+      if (dof[(size_t)i * nn + n] > 0) grp[n] = gid[owner[dof[(size_t)i * nn + n] - 1]];
+  std::vector<int> off((size_t)ng + 1), two((size_t)3 * ng), so((size_t)ng + 1), eo((size_t)ng + 1);
+  int *d_grp = nullptr, *d_two = nullptr, *d_err = nullptr, *d_off = nullptr;
+  int4 *d_row = nullptr;
+  auto done = [&](int r) {
+    for (void *p : {(void *)d_grp, (void *)d_two, (void *)d_err, (void *)d_off, (void *)d_row})
+      if (p) cudaFree(p);
+    return r;
+  };
+  if (cudaMalloc(&d_grp, sizeof(int) * nn) || cudaMalloc(&d_two, sizeof(int) * 3 * ng) ||
+      cudaMalloc(&d_err, sizeof(int)) || cudaMalloc(&d_off, sizeof(int) * 2 * (ng + 1)) ||
+      cudaMalloc(&d_row, sizeof(int4) * ng)) {
+    cudaGetLastError();
+    return done(PGFEM_GPU_ENOMEM);
+  }
+  const unsigned b4 = (unsigned)((4 * ne + 255) / 256), bg = (unsigned)((ng + 127) / 128);
+  cudaStream_t s = c->stream;
+  auto bad = [](cudaError_t e) { return e != cudaSuccess; };
+  const cudaMemcpyKind up = cudaMemcpyHostToDevice, down = cudaMemcpyDeviceToHost;
+  if (bad(cudaMemcpyAsync(d_grp, grp.data(), sizeof(int) * nn, up, s)) ||
+      bad(cudaMemcpyAsync(d_row, row.data(), sizeof(int4) * ng, up, s)) ||
+      bad(cudaMemsetAsync(d_two, 0, sizeof(int) * ng, s)) || bad(cudaMemsetAsync(d_err, 0, sizeof(int), s)))
+    return done(PGFEM_GPU_ECUDA);
+  k_gather_count<<<b4, 256, 0, s>>>(c->conn, ne, d_grp, d_two);
+  if (bad(cudaMemcpyAsync(two.data(), d_two, sizeof(int) * ng, down, s)) || bad(cudaStreamSynchronize(s)))
+    return done(PGFEM_GPU_ECUDA);
+  int most = 0;
+  for (long g = 0; g < ng; g++) {
+    off[g + 1] = off[g] + two[g];
+    most = std::max(most, two[g]);
+  }
+  if (most > kGatherMost) return done(PGFEM_GPU_OK);
+  int r, *inc = nullptr;
+  if ((r = dalloc(c, &inc, off[ng]))) return done(r);
+  c->g_mem[0] = inc;
+  if (bad(cudaMemcpyAsync(d_off, off.data(), sizeof(int) * (ng + 1), up, s)) ||
+      bad(cudaMemsetAsync(d_two, 0, sizeof(int) * ng, s)))
+    return done(PGFEM_GPU_ECUDA);
+  k_gather_fill<<<b4, 256, 0, s>>>(c->conn, ne, d_grp, d_off, d_two, inc);
+  k_gather_columns<<<bg, 128, 0, s>>>(ng, c->conn, ne, c->mask, c->pos, d_off, inc, d_row, 0, nullptr, d_two, nullptr,
+                                      nullptr, 0, d_err);
+  int err = 0;
+  if (bad(cudaMemcpyAsync(two.data(), d_two, sizeof(int) * 3 * ng, down, s)) ||
+      bad(cudaMemcpyAsync(&err, d_err, sizeof(int), down, s)) || bad(cudaStreamSynchronize(s)))
+    return done(PGFEM_GPU_ECUDA);
+  long tot = 0;
+  for (long g = 0; g < ng; g++) tot += two[ng + g];
+  if (err || tot > 0x7fffffffL) return done(PGFEM_GPU_OK);
+  GatherLists gl;
+  gl.ng = ng;
+  gl.most = most;
+  std::vector<int4> head((size_t)2 * ng);
+  for (long g = 0; g < ng; g++) {
+    const int n = off[g + 1] - off[g], ns = two[g], npk = two[ng + g];
+    so[g + 1] = so[g] + ns;
+    eo[g + 1] = eo[g] + npk;
+    gl.slots = std::max(gl.slots, ns);
+    gl.packs = std::max(gl.packs, npk);
+    gl.width = std::max(gl.width, row[g].y);
+    head[2 * g] = make_int4(off[g], so[g], eo[g], row[g].x);
+    head[2 * g + 1] = make_int4(n | ns << 8 | npk << 16 | row[g].w << 28, row[g].y, row[g].z, two[2 * ng + g]);
+  }
+  // the CTAs of every schedule (up to four warps) have to fit the shared memory
+  if (4 * (size_t)gather_plan(c->model, most, gl.slots, gl.packs, gl.width).bytes > (size_t)kGatherSmem)
+    return done(PGFEM_GPU_OK);
+  int4 *d_head = nullptr;
+  uint2 *d_slot = nullptr;
+  uint2 *d_ent = nullptr;
+  if ((r = upload(c, &d_head, head.data(), head.size()))) return done(r);
+  c->g_mem[1] = d_head;
+  if ((r = dalloc(c, &d_slot, so[ng]))) return done(r);
+  c->g_mem[2] = d_slot;
+  if ((r = dalloc(c, &d_ent, eo[ng]))) return done(r);
+  c->g_mem[3] = d_ent;
+  k_gather_columns<<<bg, 128, 0, s>>>(ng, c->conn, ne, c->mask, c->pos, d_off, inc, d_row, 1, d_head, nullptr, d_slot,
+                                      d_ent, gather_zero(most), d_err);
+  if (bad(cudaGetLastError()) || bad(cudaStreamSynchronize(s))) return done(PGFEM_GPU_ECUDA);
+  if (c->model != PGFEM_MODEL_CP && (r = dalloc(c, &c->p1rec, (size_t)kP1Rec * ne))) return done(r);
+  gl.head = d_head;
+  gl.inc = inc;
+  gl.slot = d_slot;
+  gl.ent = d_ent;
+  c->gl = gl;
+  c->gather = true;
+  return done(PGFEM_GPU_OK);
+}
+
 // Greedy colouring: elements of one colour share no node, so their R and K
 // updates touch disjoint rows and need no atomics.
 // Greedy element colours for the plain-add scatter: no two elements of one
 // colour share a free DOF, i.e. a row of R and K.  (Periodic meshes map
 // distinct slave and master nodes to one DOF, so sharing no node is not
 // enough.)
-void build_colours(const pgfem_mesh_desc *m, std::vector<int> &elems, std::vector<long> &off) {
+// conn[nne][ne] and dof[3][nn] as the context holds them.
+void build_colours(const pgfem_gpu_ctx *m, const std::vector<int> &conn, const std::vector<int> &dof,
+                   std::vector<int> &elems, std::vector<long> &off) {
   std::vector<int> colour(m->ne, -1);
   std::vector<std::vector<uint8_t>> used;
   int ncol = 0;
   auto dof_of = [&](long e, int a, int k) {  // 1-based free DOF id, 0 for fixed / prescribed
-    const long id = m->dof_id[(long)m->conn[e * m->nne + a] * 3 + k];
+    const long id = dof[(size_t)k * m->nn + conn[(size_t)a * m->ne + e]];
     return id > 0 && id <= m->ndof ? id : 0L;
   };
   for (long e = 0; e < m->ne; e++) {
@@ -1119,6 +1325,8 @@ int pgfem_gpu_create(const pgfem_mesh_desc *m, const pgfem_material_desc *mat, c
     if (ce != cudaSuccess) return fail(PGFEM_GPU_ECUDA);
     if (herr) return fail(PGFEM_GPU_EPATTERN);
   }
+  // linear tets: lists of the row owners
+  if (m->nne == 4 && c->mat.dev_pot != 2 && (r = build_gather(c, dof, rowptr0, rowlen, mask))) return fail(r);
   // tensor-core quadratic-tet path: processing order, scatter blocks in that
   // order, the second stream that zeroes K
   if (m->nne == 10 && c->model != PGFEM_MODEL_CP && c->mat.dev_pot != 2) {
@@ -1145,7 +1353,7 @@ int pgfem_gpu_create(const pgfem_mesh_desc *m, const pgfem_material_desc *mat, c
         (r = dalloc(c, &c->cp_detJw, ne)) || (r = dalloc(c, &c->cp_out, (size_t)kCpOut * c->nqp)) ||
         (r = dalloc(c, &c->cp_iters, c->nqp)) || (r = dalloc(c, &c->cp_counter, 1)) ||
         (r = dalloc(c, &c->cp_fallbacks, 1)) || (r = dalloc(c, &c->cp_conv, c->nqp)) ||
-        (c->cp_rot && (r = dalloc(c, &c->cp_rec, (size_t)kCxRec * kCxTile * ((ne + kCxTile - 1) / kCxTile)))))
+        (c->cp_rot && (r = dalloc(c, &c->cp_rec, (size_t)kCxRec * ne))))
       return fail(r);
     std::vector<double> Fn((size_t)9 * c->nqp, 0.0);  // F at t_n: identity until the first commit
     for (long q = 0; q < c->nqp; q++) Fn[0 * c->nqp + q] = Fn[4 * c->nqp + q] = Fn[8 * c->nqp + q] = 1.0;
@@ -1167,13 +1375,6 @@ int pgfem_gpu_create(const pgfem_mesh_desc *m, const pgfem_material_desc *mat, c
       cudaMemcpyAsync(c->state_nm1, s0.data(), s0.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream);
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) return fail(PGFEM_GPU_ECUDA);
   }
-  // colours for the deterministic scatter mode
-  {
-    std::vector<int> el;
-    build_colours(m, el, c->colour_off);
-    if ((r = upload(c, &c->colour_elems, el.data(), el.size()))) return fail(r);
-    if (cudaStreamSynchronize(c->stream) != cudaSuccess) return fail(PGFEM_GPU_ECUDA);
-  }
   *out = c;
   return PGFEM_GPU_OK;
 }
@@ -1188,6 +1389,15 @@ int pgfem_gpu_destroy(pgfem_gpu_ctx *c) {
 
 int pgfem_gpu_set_scatter_mode(pgfem_gpu_ctx *c, int mode) {
   if (!c || (mode != PGFEM_SCATTER_ATOMIC && mode != PGFEM_SCATTER_COLOUR)) return PGFEM_GPU_EINVAL;
+  if (mode == PGFEM_SCATTER_COLOUR && !c->colour_elems) {  // the colours, on first use
+    std::vector<int> conn((size_t)c->nne * c->ne), dof((size_t)3 * c->nn), el;
+    CK(cudaMemcpyAsync(conn.data(), c->conn, sizeof(int) * conn.size(), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(dof.data(), c->dof, sizeof(int) * dof.size(), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    build_colours(c, conn, dof, el, c->colour_off);
+    if (int r = upload(c, &c->colour_elems, el.data(), el.size())) return r;
+    CK(cudaStreamSynchronize(c->stream));
+  }
   c->scatter_mode = mode;
   return PGFEM_GPU_OK;
 }
@@ -1415,8 +1625,8 @@ int pgfem_gpu_launches_per_assembly(const pgfem_gpu_ctx *c) {
     return 1 + (c->scatter_mode == PGFEM_SCATTER_COLOUR ? (int)c->colour_off.size() - 1 : 1) + nbc;
   if (c->nne == 10 && c->scatter_mode == PGFEM_SCATTER_ATOMIC)
     return 3 + nbc;  // u expansion, point updates, tensor-core R+K assembly
-  if (c->nne == 4 && c->scatter_mode == PGFEM_SCATTER_ATOMIC)
-    return 3 + nbc;  // u expansion, point updates, column-split R+K assembly
+  if (c->nne == 4 && c->scatter_mode == PGFEM_SCATTER_ATOMIC)  // (u expansion,) point updates, R+K assembly
+    return (c->gather && !c->nbc_nface ? 2 : 3) + nbc;
   const int nasm = c->scatter_mode == PGFEM_SCATTER_COLOUR ? (int)c->colour_off.size() - 1 : 1;
   return 1 + nasm + nbc;  // u expansion + assembly launches (memsets are not kernels of ours)
 }
