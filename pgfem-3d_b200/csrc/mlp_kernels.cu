@@ -4,8 +4,8 @@
 // the gradient accumulator, the packed BF16 weights / FP32 biases that the
 // tcgen05 kernels stage into shared memory, and the feature/target scaling.
 // Training runs entirely on the GPU with this file's kernels: per step one
-// k_mlp_train launch (one CTA per 128-sample tile, fused forward + backward,
-// gradients reduced with FP32 atomics) and one k_mlp_adam launch.
+// k_mlp_train launch (CTAs over 128-sample tiles, fused forward + backward, a copy
+// of the gradient vector per CTA) and one k_mlp_adam launch that adds the copies.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -27,6 +27,12 @@ struct pgfem_mlp {
   float *bias = nullptr, *scale = nullptr;
   unsigned *err = nullptr;
   double *loss = nullptr;
+  // workspaces of training, kept between calls: gradient copies, shuffled order,
+  // epoch losses
+  float *part = nullptr;
+  int *perm = nullptr;
+  double *losses = nullptr;
+  long part_n = 0, perm_n = 0, losses_n = 0;
   float h_scale[kScale];
   long adam_t = 0;
   uint64_t wait_ns = pgb::mlp::kWaitNs;
@@ -86,7 +92,7 @@ int num_sms() {
 }
 
 int pack(pgfem_mlp *m) {
-  k_mlp_adam<<<(kNParam + 255) / 256, 256>>>(m->params, m->grad, m->mom, m->vel, m->w, m->bias, 0.f, 0.f, 0.f,
+  k_mlp_adam<<<(kNParam + 255) / 256, 256>>>(m->params, nullptr, 0, m->mom, m->vel, m->w, m->bias, 0.f, 0.f, 0.f,
                                              0.f, 0.f, 0.f, 0);
   MCK(cudaGetLastError());
   return PGFEM_GPU_OK;
@@ -103,13 +109,32 @@ int read_err(pgfem_mlp *m) {
   return PGFEM_GPU_OK;
 }
 
-// launches the tiles of one gradient evaluation over rows perm[first .. first+count)
+// grows a device workspace of n elements
+template <class T>
+int grow(T **p, long *have, long n) {
+  if (*have >= n) return PGFEM_GPU_OK;
+  cudaFree(*p);
+  *p = nullptr;
+  *have = 0;
+  if (cudaMalloc(p, sizeof(T) * n) != cudaSuccess) {
+    cudaGetLastError();
+    return PGFEM_GPU_ENOMEM;
+  }
+  *have = n;
+  return PGFEM_GPU_OK;
+}
+
+// CTAs (gradient copies) of a gradient evaluation over `count` rows
+int grad_parts(long count) { return (int)std::min<long>((count + kTile - 1) / kTile, num_sms()); }
+
+// launches the tiles of one gradient evaluation over rows perm[first .. first+count):
+// grad_parts(count) copies in m->part
 int launch_grad(pgfem_mlp *m, long count, long first, const int *perm, const float *x, const float *t,
                 float inv_batch, cudaStream_t s) {
-  const long tiles = (count + kTile - 1) / kTile;
-  if (tiles > 0x7fffffffL) return PGFEM_GPU_ELIMIT;
-  k_mlp_train<<<(unsigned)tiles, kThreads, kTrainSmem, s>>>(m->dev_view(), count, first, perm, x, t, inv_batch,
-                                                            m->grad, m->loss);
+  const int np = grad_parts(count);
+  if (int r = grow(&m->part, &m->part_n, (long)np * kNParam)) return r;
+  k_mlp_train<<<(unsigned)np, kTrainThreads, kTrainSmem, s>>>(m->dev_view(), count, first, perm, x, t, inv_batch,
+                                                             m->part, m->loss);
   MCK(cudaGetLastError());
   return PGFEM_GPU_OK;
 }
@@ -174,6 +199,9 @@ int pgfem_mlp_destroy(pgfem_mlp *m) {
   cudaFree(m->scale);
   cudaFree(m->err);
   cudaFree(m->loss);
+  cudaFree(m->part);
+  cudaFree(m->perm);
+  cudaFree(m->losses);
   delete m;
   return PGFEM_GPU_OK;
 }
@@ -272,7 +300,7 @@ int pgfem_mlp_predict_device(pgfem_mlp *m, long n, const float *d_x, float *d_y,
   pgb::mlp::MlpDev dv = m->dev_view();
   dv.stall = m->stall;
   m->stall = 0;
-  k_mlp_forward<<<grid, kThreads, kInfSmem, (cudaStream_t)stream>>>(dv, n, d_x, d_y);
+  k_mlp_forward<<<grid, kInfThreads, kInfSmem, (cudaStream_t)stream>>>(dv, n, d_x, d_y);
   MCK(cudaGetLastError());
   return PGFEM_GPU_OK;
 }
@@ -307,14 +335,17 @@ int pgfem_mlp_loss_grad(pgfem_mlp *m, long n, const float *x, const float *t, fl
   int r = PGFEM_GPU_OK;
   if (cudaMemcpy(dx, x, sizeof(float) * n * kIn, cudaMemcpyHostToDevice) ||
       cudaMemcpy(dt, t, sizeof(float) * n * kOut, cudaMemcpyHostToDevice) ||
-      cudaMemset(m->grad, 0, sizeof(float) * kNParam) || cudaMemset(m->loss, 0, sizeof(double)))
+      cudaMemset(m->loss, 0, sizeof(double)))
     r = PGFEM_GPU_ECUDA;
   if (!r) r = set_smem_attrs();
   if (!r) r = launch_grad(m, n, 0, nullptr, dx, dt, 1.0f / (float)n, nullptr);
+  if (!r) {
+    k_mlp_reduce<<<(kNParam + 255) / 256, 256>>>(m->part, grad_parts(n), m->grad);
+    if (cudaGetLastError()) r = PGFEM_GPU_ECUDA;
+  }
   if (!r && (cudaMemcpy(grad, m->grad, sizeof(float) * kNParam, cudaMemcpyDeviceToHost) ||
              (loss && cudaMemcpy(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost))))
     r = PGFEM_GPU_ECUDA;
-  cudaMemset(m->grad, 0, sizeof(float) * kNParam);
   cudaFree(dx);
   cudaFree(dt);
   if (!r) r = read_err(m);
@@ -327,22 +358,20 @@ int pgfem_mlp_train_device(pgfem_mlp *m, long n, const float *d_x, const float *
   if (n > 0x7fffffffL) return PGFEM_GPU_ELIMIT;
   int r = set_smem_attrs();
   if (r) return r;
-  int *perm = nullptr;
-  double *losses = nullptr;
-  if (cudaMalloc(&perm, sizeof(int) * n) || cudaMalloc(&losses, sizeof(double) * std::max(1, o->epochs))) {
-    cudaGetLastError();
-    cudaFree(perm);
-    return PGFEM_GPU_ENOMEM;
-  }
+  if ((r = grow(&m->perm, &m->perm_n, n)) || (r = grow(&m->losses, &m->losses_n, std::max(1, o->epochs)))) return r;
+  int *perm = m->perm;
+  double *losses = m->losses;
   std::vector<int> h(n);
   uint64_t st = o->seed;
   const long nb = n / o->batch;  // full batches per epoch (the remainder rotates with the shuffle)
   const long total = (long)o->epochs * std::max<long>(nb, 1);
   long step = 0;
-  cudaMemset(m->grad, 0, sizeof(float) * kNParam);
   for (int ep = 0; ep < o->epochs && !r; ep++) {
     for (long i = 0; i < n; i++) h[i] = (int)i;
-    for (long i = n - 1; i > 0; i--) std::swap(h[i], h[(long)(uniform01(st) * (double)(i + 1)) % (i + 1)]);
+    for (long i = n - 1; i > 0; i--) {
+      const long j = (long)(uniform01(st) * (double)(i + 1));
+      std::swap(h[i], h[j > i ? 0 : j]);  // the product can round up to i + 1
+    }
     if (cudaMemcpy(perm, h.data(), sizeof(int) * n, cudaMemcpyHostToDevice) ||
         cudaMemset(m->loss, 0, sizeof(double))) {
       r = PGFEM_GPU_ECUDA;
@@ -359,8 +388,8 @@ int pgfem_mlp_train_device(pgfem_mlp *m, long n, const float *d_x, const float *
       m->adam_t++;
       const float c1 = (float)(1.0 / (1.0 - std::pow((double)o->beta1, (double)m->adam_t)));
       const float c2 = (float)(1.0 / (1.0 - std::pow((double)o->beta2, (double)m->adam_t)));
-      k_mlp_adam<<<(kNParam + 255) / 256, 256>>>(m->params, m->grad, m->mom, m->vel, m->w, m->bias, lr, o->beta1,
-                                                 o->beta2, o->eps, c1, c2, 1);
+      k_mlp_adam<<<(kNParam + 255) / 256, 256>>>(m->params, m->part, grad_parts(cnt), m->mom, m->vel, m->w, m->bias,
+                                                 lr, o->beta1, o->beta2, o->eps, c1, c2, 1);
       if (cudaGetLastError()) r = PGFEM_GPU_ECUDA;
     }
     // mean batch loss of the epoch
@@ -373,8 +402,6 @@ int pgfem_mlp_train_device(pgfem_mlp *m, long n, const float *d_x, const float *
     if (cudaMemcpy(hl.data(), losses, sizeof(double) * o->epochs, cudaMemcpyDeviceToHost)) r = PGFEM_GPU_ECUDA;
     for (int ep = 0; ep < o->epochs && !r; ep++) epoch_loss[ep] = hl[ep] / (double)std::max<long>(nb, 1);
   }
-  cudaFree(perm);
-  cudaFree(losses);
   if (!r) r = read_err(m);
   return r;
 }

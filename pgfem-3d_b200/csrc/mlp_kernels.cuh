@@ -48,13 +48,18 @@ constexpr int kScale = 80;
 // shared-memory byte offsets (all multiples of 128)
 constexpr uint32_t sW1 = 0, sW2 = sW1 + kH * kInP * 2, sW3 = sW2 + kH * kH * 2, sW4 = sW3 + kH * kH * 2,
                    sX0 = sW4 + kOutP * kH * 2, sH1 = sX0 + kTile * kInP * 2;
-// inference: one activation buffer reused layer to layer
-constexpr uint32_t sInfBias = sH1 + kTile * kH * 2, sInfScale = sInfBias + kNPB * 4,
-                   sInfMisc = sInfScale + kScale * 4, kInfSmem = sInfMisc + 64;
+// inference: kSlots tiles in flight per CTA, eight warps each (a TMEM lane quarter
+// and half of the columns a warp); per slot a feature buffer and one activation
+// buffer reused layer to layer
+constexpr int kSlots = 3, kSlotThreads = 256, kInfThreads = kSlots * kSlotThreads;
+constexpr uint32_t kSlotBytes = (sH1 - sX0) + kTile * kH * 2, sInfBias = sX0 + kSlots * kSlotBytes,
+                   sInfScale = sInfBias + kNPB * 4, sInfMisc = sInfScale + kScale * 4, kInfSmem = sInfMisc + 128;
+static_assert(kInfSmem <= 232448, "inference slots exceed the 227 KB shared-memory limit");
 // training: H1, H2, H3 kept for the weight gradients, one error-term buffer
 constexpr uint32_t sH2 = sH1 + kTile * kH * 2, sH3 = sH2 + kTile * kH * 2, sDZ = sH3 + kTile * kH * 2,
                    sTrBias = sDZ + kTile * kH * 2, sTrScale = sTrBias + kNPB * 4,
                    sTrMisc = sTrScale + kScale * 4, kTrainSmem = sTrMisc + 64;
+constexpr int kTrainThreads = 512;  // sixteen warps: a TMEM lane quarter and a quarter of the columns each
 static_assert(kTrainSmem <= 232448, "training tile exceeds the 227 KB shared-memory limit");
 
 struct MlpDev {
@@ -134,8 +139,8 @@ __device__ __forceinline__ void mbar_init(uint32_t a, uint32_t count) {
 
 // Bounded wait for the completion of phase `parity`; false after `limit` ns.
 __device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity, uint64_t limit) {
-  const uint64_t t0 = gtimer();
-  for (;;) {
+  uint64_t t0 = 0;
+  for (int spin = 0;; spin++) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -144,7 +149,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity, uint64_t 
         : "r"(a), "r"(parity)
         : "memory");
     if (ok) return true;
-    if (gtimer() - t0 > limit) return false;
+    if (spin == 0) t0 = gtimer();
+    else if (gtimer() - t0 > limit) return false;
   }
 }
 
@@ -224,111 +230,166 @@ __device__ __forceinline__ void load_params(unsigned char *sm, const MlpDev &m, 
   for (int i = threadIdx.x; i < kScale; i += blockDim.x) ss[i] = m.scale[i];
 }
 
-// one normalised feature row (34 + zero padding to 48) of tile row r
-__device__ __forceinline__ void load_x_row(unsigned char *sX, int r, const float *xrow, const float *ss) {
-  float v[kInP];
-#pragma unroll
-  for (int j = 0; j < kInP; j++) v[j] = (xrow && j < kIn) ? (xrow[j] - ss[j]) * ss[kIn + j] : 0.0f;
-#pragma unroll
-  for (int c = 0; c < kInP; c += 8) st8(sX, r, c, kInP, v + c);
-}
-
-// hidden-layer epilogue: rows of this thread, H = GELU(Z + b) -> blocked BF16
-__device__ __forceinline__ void epi_hidden(uint32_t tz, unsigned char *sHout, int r, const float *bias) {
-#pragma unroll 1
-  for (int c0 = 0; c0 < kH; c0 += 16) {
-    float v[16];
-    tmem_ld16(tz + (uint32_t)c0, v);
-#pragma unroll
-    for (int i = 0; i < 16; i++) v[i] = gelu(v[i] + bias[c0 + i]);
-    st8(sHout, r, c0, kH, v);
-    st8(sHout, r, c0 + 8, kH, v + 8);
-  }
-}
-
 // ------------------------------------------------------------- inference --
 // Persistent over tiles of 128 points: y[n][12] = network(x[n][34]) in raw units.
-__global__ void __launch_bounds__(kThreads, 1)
+// Three tiles are in flight per CTA (eight warps, 128 TMEM columns, an mbarrier and
+// a named barrier each) over one copy of the weights, so that one tile's chain
+// and loads run under the others' epilogues; a slot's next features are loaded
+// into registers beside its layers.  Bound by the GELU epilogues: erff and the
+// rounding around it are some 29 instructions a value, 0.21 ms of issue slots at
+// 663,552 points.  Measured there: one tile of four warps a CTA 480 us, three slots of
+// four warps 354, of eight 305 (chunks of 16 columns; of 32 the registers spill,
+// 339).  A shorter erf (0.26 ms) changes BF16 roundings of the activations and with
+// them the output by 1e-4, so erff stays.
+__device__ __forceinline__ void slot_sync(int slot) {
+  asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "n"(kSlotThreads) : "memory");
+}
+
+__global__ void __launch_bounds__(kInfThreads, 1)
     k_mlp_forward(const MlpDev m, long n, const float *__restrict__ x, float *__restrict__ y) {
   extern __shared__ __align__(128) unsigned char sm[];
   float *sb = reinterpret_cast<float *>(sm + sInfBias);
   float *ss = reinterpret_cast<float *>(sm + sInfScale);
-  uint64_t *mbar = reinterpret_cast<uint64_t *>(sm + sInfMisc);
-  uint32_t *slot = reinterpret_cast<uint32_t *>(sm + sInfMisc + 8);
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const uint32_t ab = smem_u32(sm), mb = smem_u32(mbar);
-  if (warp == 0) tmem_alloc(smem_u32(slot), 128);
-  if (tid == 0) mbar_init(mb, 1);
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + sInfMisc + 64);
+  const int tid = threadIdx.x, warp = tid >> 5, slot = warp >> 3, st = tid & (kSlotThreads - 1);
+  const int half = (warp >> 2) & 1, lrow = st & (kTile - 1);  // columns 64 half .. 64 half + 63 of tile row lrow
+  const uint32_t ab = smem_u32(sm), mb = ab + sInfMisc + 8u * (uint32_t)slot;
+  int *sfail = reinterpret_cast<int *>(sm + sInfMisc + 32) + slot;
+  if (warp == 0) tmem_alloc(smem_u32(tslot), 512);
+  if (st == 0) {
+    mbar_init(mb, 1);
+    *sfail = 0;
+  }
   load_params(sm, m, sb, ss);
+  const uint32_t oX = sX0 + (uint32_t)slot * kSlotBytes, oH = oX + (sH1 - sX0);
+  for (int i = st; i < kTile * kInP * 2 / 16; i += kSlotThreads)  // columns 34..47 stay zero
+    *reinterpret_cast<uint4 *>(sm + oX + 16 * i) = make_uint4(0u, 0u, 0u, 0u);
   tc_before();
   __syncthreads();
   tc_after();
-  const uint32_t tbase = *slot;
-  const uint32_t tme = tbase + ((uint32_t)(warp * 32) << 16);  // this warp's lane quarter, column 0
-  const long ntiles = (n + kTile - 1) / kTile;
+  const uint32_t tbase = *tslot + 128u * (uint32_t)slot;
+  const uint32_t tme = tbase + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's lane quarter, column 0
+  const long ntiles = (n + kTile - 1) / kTile, step = (long)gridDim.x * kSlots;
+  const bool x8 = (reinterpret_cast<uintptr_t>(x) & 7) == 0, y16 = (reinterpret_cast<uintptr_t>(y) & 15) == 0;
   uint32_t phase = 0;
   bool fail = false;
   constexpr uint32_t ID_H = idesc_bf16(128, kH, 0, 0), ID_O = idesc_bf16(128, kOutP, 0, 0);
-  for (long t = blockIdx.x; t < ntiles && !fail; t += gridDim.x) {
-    const long row = t * kTile + tid;
-    load_x_row(sm + sX0, tid, row < n ? x + row * kIn : nullptr, ss);
+  constexpr int kPairs = kIn / 2;  // a tile's rows are contiguous: 128 x 17 pairs
+  constexpr int kFetch = (kTile * kPairs + kSlotThreads - 1) / kSlotThreads;
+  float2 xr[kFetch];
+  auto fetch = [&](long t) {
+    const float *p = x + t * kTile * kIn;
+    const long rows = n - t * kTile, left = (rows < kTile ? rows : kTile) * kPairs;  // pairs of the tile's rows below n
+#pragma unroll
+    for (int k = 0; k < kFetch; k++) {
+      const int i = st + k * kSlotThreads;
+      float2 v = make_float2(0.0f, 0.0f);
+      if (i < left) {
+        if (x8) v = *reinterpret_cast<const float2 *>(p + 2 * i);
+        else v = make_float2(p[2 * i], p[2 * i + 1]);
+      }
+      xr[k] = v;
+    }
+  };
+  const long t0 = blockIdx.x + (long)slot * gridDim.x;
+  if (t0 < ntiles) fetch(t0);
+  for (long t = t0; t < ntiles && !fail; t += step) {
+#pragma unroll
+    for (int k = 0; k < kFetch; k++) {
+      const int i = st + k * kSlotThreads, r = i / kPairs, c = 2 * (i - r * kPairs);
+      if (i >= kTile * kPairs) break;
+      const float2 mu = *reinterpret_cast<const float2 *>(ss + c), is = *reinterpret_cast<const float2 *>(ss + kIn + c);
+      *reinterpret_cast<uint32_t *>(sm + oX + blk_off(r, c & ~7, kInP) + 2 * (c & 7)) =
+          pack2((xr[k].x - mu.x) * is.x, (xr[k].y - mu.y) * is.y);
+    }
     fence_async_smem();
     tc_before();
-    __syncthreads();
+    slot_sync(slot);
     tc_after();
+    if (t + step < ntiles) fetch(t + step);
+    const long row = t * kTile + lrow;
     for (int l = 0; l < 4 && !fail; l++) {
-      // (with m.stall the CTA's first chain and its commit are not issued: the
-      // wait below runs out with no MMA in flight)
-      if (tid == 0 && !(m.stall && l == 0 && t == blockIdx.x)) {
+      // (with m.stall a slot's first chain and its commit are not issued: the
+      // wait below runs out with no MMA of the slot in flight)
+      if (st == 0 && !(m.stall && l == 0 && t == t0)) {
         if (l == 0)
-          mma_chain(tbase, kmajor(ab + sX0, kInP), kmajor(ab + sW1, kInP), kInP / 16, ID_H);
+          mma_chain(tbase, kmajor(ab + oX, kInP), kmajor(ab + sW1, kInP), kInP / 16, ID_H);
         else if (l < 3)
-          mma_chain(tbase, kmajor(ab + sH1, kH), kmajor(ab + (l == 1 ? sW2 : sW3), kH), kH / 16, ID_H);
+          mma_chain(tbase, kmajor(ab + oH, kH), kmajor(ab + (l == 1 ? sW2 : sW3), kH), kH / 16, ID_H);
         else
-          mma_chain(tbase, kmajor(ab + sH1, kH), kmajor(ab + sW4, kH), kH / 16, ID_O);
+          mma_chain(tbase, kmajor(ab + oH, kH), kmajor(ab + sW4, kH), kH / 16, ID_O);
         mma_commit(mb);
       }
-      const bool ok = mbar_wait(mb, phase, m.wait_ns);
+      if (!mbar_wait(mb, phase, m.wait_ns)) *sfail = 1;
       phase ^= 1;
-      if (__syncthreads_or(!ok)) {
+      slot_sync(slot);
+      if (*reinterpret_cast<volatile int *>(sfail)) {
         fail = true;
         break;
       }
       tc_after();
       if (l < 3) {
-        epi_hidden(tme, sm + sH1, tid, sb + (l == 0 ? pb1 : l == 1 ? pb2 : pb3));
-      } else {
+        const float *bias = sb + (l == 0 ? pb1 : l == 1 ? pb2 : pb3);
+#pragma unroll 1
+        for (int c0 = 64 * half; c0 < 64 * half + 64; c0 += 16) {
+          float v[16];
+          tmem_ld16(tme + (uint32_t)c0, v);
+#pragma unroll
+          for (int i = 0; i < 16; i += 4) {
+            const float4 b = *reinterpret_cast<const float4 *>(bias + c0 + i);
+            v[i] = gelu(v[i] + b.x);
+            v[i + 1] = gelu(v[i + 1] + b.y);
+            v[i + 2] = gelu(v[i + 2] + b.z);
+            v[i + 3] = gelu(v[i + 3] + b.w);
+          }
+          st8(sm + oH, lrow, c0, kH, v);
+          st8(sm + oH, lrow, c0 + 8, kH, v + 8);
+        }
+      } else if (!half) {
         float v[16];
         tmem_ld16(tme, v);  // warp-wide: every lane loads, rows past n store nothing
         if (row < n) {
 #pragma unroll
-          for (int i = 0; i < kOut; i++) y[row * kOut + i] = (v[i] + sb[pb4 + i]) * ss[2 * kIn + i];
+          for (int i = 0; i < kOut; i++) v[i] = (v[i] + sb[pb4 + i]) * ss[2 * kIn + i];
+          if (y16) {
+#pragma unroll
+            for (int i = 0; i < kOut; i += 4)
+              *reinterpret_cast<float4 *>(y + row * kOut + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < kOut; i++) y[row * kOut + i] = v[i];
+          }
         }
       }
       fence_async_smem();
       tc_before();
-      __syncthreads();
+      slot_sync(slot);
       tc_after();
     }
   }
   if (fail) {
     mbar_wait(mb, phase ^ 1u, m.wait_ns);  // bounded: let a late MMA finish before its TMEM is released
-    if (tid == 0) atomicOr(m.err, 1u);
+    if (st == 0) atomicOr(m.err, 1u);
   }
   tc_before();
   __syncthreads();
   tc_after();
-  if (warp == 0) tmem_free(tbase, 128);
+  if (warp == 0) tmem_free(*tslot, 512);
 }
 
 // -------------------------------------------------------------- training --
-// One tile of 128 samples (rows perm[first + i] of x/t, i < count): forward,
-// loss 1/(2B) sum (out - t/y_std)^2, backward; parameter gradients added to
-// grad (FP32, master layout), loss added to *loss.
-__global__ void __launch_bounds__(kThreads, 1)
+// Tiles of 128 samples (rows perm[first + i] of x/t, i < count), tile b, b + grid, ...
+// per CTA: forward, loss 1/(2B) sum (out - t/y_std)^2, backward.  A CTA keeps its
+// parameter gradients in its own copy of the vector, part[blockIdx.x] (stored by its
+// first tile, added to by later ones); k_mlp_adam and k_mlp_reduce add the copies in
+// order.  A launch of 64 tiles: 67 us; with the gradients added to one vector by
+// FP32 atomics (39 k per tile, every CTA on the same addresses) and four warps a
+// CTA 104 us.  The sums no longer depend on timing.  Bound by the serial chain of ten
+// products and their epilogues in one tile.
+__global__ void __launch_bounds__(kTrainThreads, 1)
     k_mlp_train(const MlpDev m, long count, long first, const int *__restrict__ perm,
                 const float *__restrict__ x, const float *__restrict__ tg, float inv_batch,
-                float *__restrict__ grad, double *__restrict__ loss) {
+                float *__restrict__ part, double *__restrict__ loss) {
   extern __shared__ __align__(128) unsigned char sm[];
   float *sb = reinterpret_cast<float *>(sm + sTrBias);
   float *ss = reinterpret_cast<float *>(sm + sTrScale);
@@ -336,21 +397,16 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint32_t *slot = reinterpret_cast<uint32_t *>(sm + sTrMisc + 8);
   double *red = reinterpret_cast<double *>(sm + sTrMisc + 16);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int r = (warp & 3) * 32 + lane, cg = warp >> 2;  // tile row (TMEM lane), column quarter
   const uint32_t ab = smem_u32(sm), mb = smem_u32(mbar);
   if (warp == 0) tmem_alloc(smem_u32(slot), 512);
   if (tid == 0) mbar_init(mb, 1);
   load_params(sm, m, sb, ss);
-  __syncthreads();  // the feature scaling in ss is read by every row below
-  const long i_row = (long)blockIdx.x * kTile + tid;
-  const bool valid = i_row < count;
-  const long src = valid ? (perm ? (long)perm[first + i_row] : first + i_row) : 0;
-  load_x_row(sm + sX0, tid, valid ? x + src * kIn : nullptr, ss);
-  fence_async_smem();
   tc_before();
-  __syncthreads();
+  __syncthreads();  // the feature scaling in ss is read by every row below
   tc_after();
   const uint32_t tbase = *slot;
-  const uint32_t lq = (uint32_t)(warp * 32) << 16;
+  const uint32_t lq = (uint32_t)((warp & 3) * 32) << 16;
   // TMEM columns: Z1 [0,128) Z2 [128,256) Z3 [256,384) scratch S [384,512)
   const uint32_t cZ1 = 0, cZ2 = 128, cZ3 = 256, cS = 384;
   uint32_t phase = 0;
@@ -358,6 +414,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   constexpr uint32_t ID_KK = idesc_bf16(128, kH, 0, 0), ID_KK_O = idesc_bf16(128, kOutP, 0, 0);
   constexpr uint32_t ID_MM_O = idesc_bf16(128, kOutP, 1, 1), ID_MM = idesc_bf16(128, kH, 1, 1);
   constexpr uint32_t ID_MM_IN = idesc_bf16(128, kInP, 1, 1), ID_KM = idesc_bf16(128, kH, 0, 1);
+  float *P = part + (long)blockIdx.x * kNParam;
+  bool valid = false, add = false;
   auto sync_all = [&]() {
     fence_async_smem();
     tc_before();
@@ -371,37 +429,78 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_after();
     return true;
   };
+  auto out1 = [&](int i, float v) { P[i] = add ? P[i] + v : v; };
+  // column sums of the error terms, row by row
   auto bias_grad = [&](int C, int nvalid, int og) {
-    __syncthreads();
     if (tid < nvalid) {
       float s = 0.0f;
-      for (int r = 0; r < kTile; r++) s += ld_blk(sm + sDZ, r, tid, C);
-      atomicAdd(grad + og + tid, s);
+#pragma unroll 16
+      for (int k = 0; k < kTile; k++) s += ld_blk(sm + sDZ, k, tid, C);
+      out1(og + tid, s);
     }
   };
-  // dW rows: this thread's TMEM lane = output neuron `tid`, columns = inputs
-  auto dw_rows = [&](uint32_t col, int kvalid, int ow) {
-    for (int c0 = 0; c0 < (kvalid + 15) / 16 * 16; c0 += 16) {
+  // dW rows: this thread's TMEM lane = output neuron r, columns = inputs
+  auto dw_rows = [&](uint32_t col, int ow) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int c0 = cg * 32 + h * 16;
       float v[16];
       tmem_ld16(tbase + lq + col + (uint32_t)c0, v);
+      float4 *o = reinterpret_cast<float4 *>(P + ow + r * kH + c0);
 #pragma unroll
-      for (int i = 0; i < 16; i++)
-        if (c0 + i < kvalid) atomicAdd(grad + ow + tid * kvalid + c0 + i, v[i]);
+      for (int i = 0; i < 4; i++) {
+        float4 w = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        if (add) {
+          const float4 p = o[i];
+          w = make_float4(w.x + p.x, w.y + p.y, w.z + p.z, w.w + p.w);
+        }
+        o[i] = w;
+      }
+    }
+  };
+  // H = GELU(Z + b) of this thread's columns
+  auto epi_h = [&](uint32_t cz, unsigned char *out, const float *bias) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int c0 = cg * 32 + h * 16;
+      float v[16];
+      tmem_ld16(tbase + lq + cz + (uint32_t)c0, v);
+#pragma unroll
+      for (int i = 0; i < 16; i++) v[i] = gelu(v[i] + bias[c0 + i]);
+      st8(out, r, c0, kH, v);
+      st8(out, r, c0 + 8, kH, v + 8);
     }
   };
   // dZ_l = (dH . W_{l+1}) * GELU'(Z_l + b_l) -> sDZ (blocked BF16, 128 columns)
   auto epi_dz = [&](uint32_t cz, const float *bias) {
-    for (int c0 = 0; c0 < kH; c0 += 16) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int c0 = cg * 32 + h * 16;
       float dh[16], z[16];
       tmem_ld16(tbase + lq + cS + (uint32_t)c0, dh);
       tmem_ld16(tbase + lq + cz + (uint32_t)c0, z);
 #pragma unroll
       for (int i = 0; i < 16; i++) dh[i] = valid ? dh[i] * gelu_d(z[i] + bias[c0 + i]) : 0.0f;
-      st8(sm + sDZ, tid, c0, kH, dh);
-      st8(sm + sDZ, tid, c0 + 8, kH, dh + 8);
+      st8(sm + sDZ, r, c0, kH, dh);
+      st8(sm + sDZ, r, c0 + 8, kH, dh + 8);
     }
   };
-  do {
+  for (long tile = blockIdx.x; tile * kTile < count && !fail; tile += gridDim.x) {
+    add = tile != blockIdx.x;
+    const long i_row = tile * kTile + r;
+    valid = i_row < count;
+    const long src = valid ? (perm ? (long)perm[first + i_row] : first + i_row) : 0;
+    if (cg < 3) {  // normalised features, 16 columns a thread
+      float v[16];
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        const int c = cg * 16 + i;
+        v[i] = valid && c < kIn ? (x[src * kIn + c] - ss[c]) * ss[kIn + c] : 0.0f;
+      }
+      st8(sm + sX0, r, cg * 16, kInP, v);
+      st8(sm + sX0, r, cg * 16 + 8, kInP, v + 8);
+    }
+    sync_all();
     // forward
     const uint32_t sHs[3] = {sH1, sH2, sH3}, sWs[3] = {sW1, sW2, sW3}, cZs[3] = {cZ1, cZ2, cZ3};
     for (int l = 0; l < 3 && !fail; l++) {
@@ -416,7 +515,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         fail = true;
         break;
       }
-      epi_hidden(tbase + lq + cZs[l], sm + sHs[l], tid, sb + (l == 0 ? pb1 : l == 1 ? pb2 : pb3));
+      epi_h(cZs[l], sm + sHs[l], sb + (l == 0 ? pb1 : l == 1 ? pb2 : pb3));
       sync_all();
     }
     if (fail) break;
@@ -428,21 +527,21 @@ __global__ void __launch_bounds__(kThreads, 1)
       fail = true;
       break;
     }
-    {  // output error terms dZ4 = (out - t/y_std) / B -> sDZ as a 128 x 16 matrix
+    if (cg == 0) {  // output error terms dZ4 = (out - t/y_std) / B -> sDZ as a 128 x 16 matrix
       float v[16];
       tmem_ld16(tbase + lq + cS, v);
       double l2 = 0.0;
 #pragma unroll
       for (int i = 0; i < 16; i++) {
-        float r = 0.0f;
+        float e = 0.0f;
         if (valid && i < kOut) {
-          r = (v[i] + sb[pb4 + i]) - tg[src * kOut + i] / ss[2 * kIn + i];
-          l2 += (double)r * (double)r;
+          e = (v[i] + sb[pb4 + i]) - tg[src * kOut + i] / ss[2 * kIn + i];
+          l2 += (double)e * (double)e;
         }
-        v[i] = r * inv_batch;
+        v[i] = e * inv_batch;
       }
-      st8(sm + sDZ, tid, 0, kOutP, v);
-      st8(sm + sDZ, tid, 8, kOutP, v + 8);
+      st8(sm + sDZ, r, 0, kOutP, v);
+      st8(sm + sDZ, r, 8, kOutP, v + 8);
       for (int o = 16; o; o >>= 1) l2 += __shfl_xor_sync(0xffffffffu, l2, o);
       if (lane == 0) red[warp] = l2;
     }
@@ -458,11 +557,11 @@ __global__ void __launch_bounds__(kThreads, 1)
       fail = true;
       break;
     }
-    {
+    if (cg == 0) {
       float v[16];
       tmem_ld16(tbase + lq + cS, v);
 #pragma unroll
-      for (int i = 0; i < kOut; i++) atomicAdd(grad + oW4 + i * kH + tid, v[i]);
+      for (int i = 0; i < kOut; i++) out1(oW4 + i * kH + r, v[i]);
     }
     sync_all();
     if (tid == 0) {  // dH3 = dZ4 W4 : M = samples, N = 128, K = 16
@@ -489,7 +588,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         fail = true;
         break;
       }
-      dw_rows(cZl[j], kH, ow[j]);
+      dw_rows(cZl[j], ow[j]);
       __syncthreads();
       epi_dz(cZprev[j], sb + pbp[j]);
       sync_all();
@@ -504,8 +603,17 @@ __global__ void __launch_bounds__(kThreads, 1)
       fail = true;
       break;
     }
-    dw_rows(cZ1, kIn, oW1);
-  } while (false);
+    if (cg < 3) {
+      float v[16];
+      tmem_ld16(tbase + lq + cZ1 + 16u * (uint32_t)cg, v);
+#pragma unroll
+      for (int i = 0; i < 16; i++)
+        if (cg * 16 + i < kIn) out1(oW1 + r * kIn + cg * 16 + i, v[i]);
+    }
+    tc_before();
+    __syncthreads();  // the next tile reuses the features and Z1
+    tc_after();
+  }
   if (fail) {
     mbar_wait(mb, phase ^ 1u, m.wait_ns);  // bounded: let a late MMA finish before its TMEM is released
     if (tid == 0) atomicOr(m.err, 1u);
@@ -516,23 +624,34 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 0) tmem_free(tbase, 512);
 }
 
-// Adam on the FP32 master vector; re-packs the BF16 weights / FP32 biases and
-// clears the gradient for the next step.
-__global__ void k_mlp_adam(float *__restrict__ p, float *__restrict__ g, float *__restrict__ mo,
+// sum of the CTAs' gradient copies of one parameter, in order
+__device__ __forceinline__ float part_sum(const float *__restrict__ part, int nparts, int i) {
+  double s = 0.0;
+#pragma unroll 16
+  for (int k = 0; k < nparts; k++) s += (double)part[(long)k * kNParam + i];
+  return (float)s;
+}
+__global__ void k_mlp_reduce(const float *__restrict__ part, int nparts, float *__restrict__ g) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < kNParam) g[i] = part_sum(part, nparts, i);
+}
+
+// Adam on the FP32 master vector with the gradient of the CTAs' copies; re-packs the
+// BF16 weights / FP32 biases.
+__global__ void k_mlp_adam(float *__restrict__ p, const float *__restrict__ part, int nparts, float *__restrict__ mo,
                            float *__restrict__ ve, __nv_bfloat16 *__restrict__ w, float *__restrict__ b,
                            float lr, float b1, float b2, float eps, float c1, float c2, int update) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= kNParam) return;
   float v = p[i];
   if (update) {
-    const float gi = g[i];
+    const float gi = part_sum(part, nparts, i);
     const float m1 = b1 * mo[i] + (1.0f - b1) * gi;
     const float v1 = b2 * ve[i] + (1.0f - b2) * gi * gi;
     mo[i] = m1;
     ve[i] = v1;
     v -= lr * (m1 * c1) / (sqrtf(v1 * c2) + eps);
     p[i] = v;
-    g[i] = 0.0f;
   }
   if (i < ob1) w[pW1 + (i / kIn) * kInP + i % kIn] = __float2bfloat16_rn(v);
   else if (i < oW2) b[pb1 + i - ob1] = v;
