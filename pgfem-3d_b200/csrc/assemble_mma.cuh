@@ -86,6 +86,7 @@ struct QpArgs {
   // three-field element (10-node records, hyperelastic and J2 models): the
   // pressure and the volume of each element (element order)
   const double *tf_P, *tf_theta;
+  double wscale;  // factor of every record's point weight (the transient's factor of K)
 };
 
 template <int NNE, int NQP, int MODEL, bool YREC = false, bool TF = false>
@@ -174,7 +175,7 @@ __global__ void __launch_bounds__(128) k_qp_update(const QpArgs A) {
     for (int j = 0; j < 3; j++)
       rec[YREC ? yrec_idx<NRF>(qs, i * 3 + j) : (i * 3 + j) * S + qs] =
           dXi[i * 3 + 0] * Fi[0 * 3 + j] + dXi[i * 3 + 1] * Fi[1 * 3 + j] + dXi[i * 3 + 2] * Fi[2 * 3 + j];
-  const double w = detJ * A.shp.w[q];
+  const double w = detJ * A.shp.w[q] * A.wscale;
   if (YREC) {
     const double h = 0.5 * t.a1 * w, c23 = (2.0 / 3.0) * w;
     // plastic point: n != 0 (the unit flow direction, s = (s : n) n)
@@ -306,7 +307,8 @@ __device__ __forceinline__ void dmma884(double &c0, double &c1, double a, double
 
 // Item (point q, column nodes b0 and b0 + 5) of one element: p_b into P, the
 // 27 values Y_q[j][(b, i, k)] of each column node and, for b0 = 0, the
-// residual rows Y_q[j][32 i + 30] = w tau_ij.  rec: the point's record fields
+// residual rows Y_q[j][32 i + 30] = w tau_ij (times rscale, the transient's ratio of
+// the residual's factor to the stiffness's, which the records carry).  rec: the point's record fields
 // with stride RS (the element's other points at rec - q + q'); shp: the
 // shape-function derivatives.
 // TF (three-field element, one pressure P and one volume theta per element):
@@ -319,7 +321,7 @@ __device__ __forceinline__ void dmma884(double &c0, double &c1, double a, double
 // Y[t][r] sits at y_idx(t, r) = tb(t) + 128 i + gk(3 b + k) for r = 32 i + 3 b + k.
 template <bool PLASTIC, int RS, bool TF = false>
 __device__ __forceinline__ void p2m_item(const double *rec, const ShapeTable &shp, int q, int b0, double *Y,
-                                         double *P, const Mat &mat) {
+                                         double *P, const Mat &mat, double rscale) {
   const double(*dN)[3] = shp.dNxi[q];
   double G[9], Tm[6], Um[6], Wm[6], s2[6], nn[6];
 #pragma unroll
@@ -428,7 +430,7 @@ __device__ __forceinline__ void p2m_item(const double *rec, const ShapeTable &sh
 #pragma unroll
     for (int j = 0; j < 3; j++)
 #pragma unroll
-      for (int i = 0; i < 3; i++) Y[tb[j] + 128 * i + 120] = Tm[vo(i, j)] - (i == j ? h - wJq * tfs : 0.0);
+      for (int i = 0; i < 3; i++) Y[tb[j] + 128 * i + 120] = rscale * (Tm[vo(i, j)] - (i == j ? h - wJq * tfs : 0.0));
   }
 }
 
@@ -512,7 +514,7 @@ __global__ void __launch_bounds__(kMThreads, 4) k_assemble_p2m(const AsmArgs arg
       const int bp = rem >> 2, q = rem & 3;
       if (e0 + el < ne) {
         p2m_item<PLASTIC, kMPts, TF>(sRec + el * NQP + q, args.shp, q, bp, sY + el * kMY, sP + el * kMP,
-                                     args.mat);
+                                     args.mat, args.rscale);
         // column offsets of node b's block inside the rows of nodes a = q, q+4, q+8
         const int *eb = sEB + (mb * TE + el) * kEBW;
         const uint16_t *pos16 = reinterpret_cast<const uint16_t *>(eb + kEBPos);
@@ -859,6 +861,149 @@ __global__ void k_tf_residual(const QpArgs A, const int *dof, double *R) {
       const int id = dof[i * A.nn + n];
       if (id > 0) atomicAdd(R + (id - 1), out[b][i]);
     }
+  }
+}
+
+// ---- three-field transient: all terms beside the newer point's assembly -------
+//
+// The transient's condensed residual is cA (fu_a + s_a Kup_a) -- the assembly at the
+// newer mid point -- plus cB fu_b + d Kup_a - f_i with d as in k_tf_transient (the
+// s_b Kup_b terms of the older point cancel) and the inertia force f_i.  One
+// thread per point forms its part of the three from the nodal fields:
+//   out_b = M dN_b/dxi - N_b e,  M_ic = cB w tau_ij G_b,cj + d w J_a G_a,ci,
+//   e = rho / (dt_np1 dt_n) w sum_C N_C v_C,  G = (dX/dxi)^-1 F^-1,
+// and the four lanes of an element add their 30 values by halving exchanges, so
+// that each ends with eight sums and their reductions.  257 us at 384,000 elements,
+// bound by the L1 wavefronts of the node loads (67 % of their peak); 96-byte node
+// records read by the lanes instead measured 326 us, as neighbouring elements no
+// longer share the sectors.
+struct TfTrResArgs {
+  const double *X, *ua, *ub, *v;  // 3*nn SoA: coordinates, u_{n+a}, u_{n-1+a}, inertia combination
+  const int *conn, *dof, *perm;
+  long nn, ne;
+  const double *mid;  // 4*ne: P_a, theta_a, P_b, theta_b
+  double *R;
+  unsigned long long *status;
+  Mat mat;
+  ShapeTable shp;
+  double cB, cR;
+};
+
+__global__ void __launch_bounds__(128, 4) k_tf_transient_terms(const TfTrResArgs A) {
+  __shared__ double sdN[4][10][3], sN[4][10], sw[4];
+  for (int i = threadIdx.x; i < 120; i += 128) (&sdN[0][0][0])[i] = A.shp.dNxi[i / 30][(i / 3) % 10][i % 3];
+  if (threadIdx.x < 40) sN[threadIdx.x / 10][threadIdx.x % 10] = A.shp.N[threadIdx.x / 10][threadIdx.x % 10];
+  if (threadIdx.x < 4) sw[threadIdx.x] = A.shp.w[threadIdx.x];
+  __syncthreads();
+  const unsigned FULL = 0xffffffffu;
+  const long t = blockIdx.x * 128L + threadIdx.x, es = t >> 2;
+  const int q = (int)(t & 3);
+  const bool in = es < A.ne;
+  const long e = in ? (A.perm ? (long)A.perm[es] : es) : 0;
+  double out[32];
+#pragma unroll
+  for (int i = 0; i < 32; i++) out[i] = 0.0;
+  double dX[9], da[9], db[9], du[3] = {0, 0, 0};
+#pragma unroll
+  for (int i = 0; i < 9; i++) dX[i] = da[i] = db[i] = 0.0;
+#pragma unroll
+  for (int b = 0; b < 10; b++) {
+    const int n = A.conn[(long)b * A.ne + e];
+    const double g0 = sdN[q][b][0], g1 = sdN[q][b][1], g2 = sdN[q][b][2], N = sN[q][b];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const double x = A.X[i * A.nn + n], ya = A.ua[i * A.nn + n], yb = A.ub[i * A.nn + n];
+      dX[i * 3] = fma(g0, x, dX[i * 3]), dX[i * 3 + 1] = fma(g1, x, dX[i * 3 + 1]), dX[i * 3 + 2] = fma(g2, x, dX[i * 3 + 2]);
+      da[i * 3] = fma(g0, ya, da[i * 3]), da[i * 3 + 1] = fma(g1, ya, da[i * 3 + 1]), da[i * 3 + 2] = fma(g2, ya, da[i * 3 + 2]);
+      db[i * 3] = fma(g0, yb, db[i * 3]), db[i * 3 + 1] = fma(g1, yb, db[i * 3 + 1]), db[i * 3 + 2] = fma(g2, yb, db[i * 3 + 2]);
+      du[i] = fma(N, A.v[i * A.nn + n], du[i]);
+    }
+  }
+  const double detJ = det3(dX);
+  double dXi[9], Fa[9], Fb[9], Fia[9], Fib[9], Ja = 0.0, Jb = 0.0;
+  const bool geo = detJ > 0.0 && inv3(dX, dXi);
+  bool oka = geo, okb = geo;
+  if (geo) {
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+      for (int j = 0; j < 3; j++) {
+        const double one = i == j ? 1.0 : 0.0;
+        Fa[i * 3 + j] = one + da[i * 3] * dXi[j] + da[i * 3 + 1] * dXi[3 + j] + da[i * 3 + 2] * dXi[6 + j];
+        Fb[i * 3 + j] = one + db[i * 3] * dXi[j] + db[i * 3 + 1] * dXi[3 + j] + db[i * 3 + 2] * dXi[6 + j];
+      }
+    Ja = det3(Fa);
+    Jb = det3(Fb);
+    oka = Ja > 0.0 && inv3(Fa, Fia);
+    okb = Jb > 0.0 && inv3(Fb, Fib);
+  }
+  const double w = geo ? detJ * sw[q] : 0.0;
+  double W = w, SJb = w * Jb;
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    W += __shfl_xor_sync(FULL, W, o);
+    SJb += __shfl_xor_sync(FULL, SJb, o);
+  }
+  const unsigned quad = 0xFu << (threadIdx.x & 28);
+  const bool geo_all = (__ballot_sync(FULL, geo) & quad) == quad;
+  const bool ok_all = (__ballot_sync(FULL, oka && okb) & quad) == quad;
+  if (in && !okb) atomicAdd(&A.status[0], 1ull);               // a point inverted at the older mid point
+  if (in && q == 0 && !ok_all) atomicAdd(&A.status[0], 1ull);  // an element inverted at either
+  double M[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, f[3] = {0, 0, 0};
+  if (geo_all)
+#pragma unroll
+    for (int i = 0; i < 3; i++) f[i] = A.cR * w * du[i];
+  if (ok_all) {
+    const double tha = A.mid[A.ne + e], Pb = A.mid[2 * A.ne + e], thb = A.mid[3 * A.ne + e], kap = A.mat.kappa;
+    double dUa, d2Ua, dUb, d2Ub, dUj, d2Uj;
+    vol_derivs(A.mat.vol_pot, tha, dUa, d2Ua);
+    vol_derivs(A.mat.vol_pot, thb, dUb, d2Ub);
+    vol_derivs(A.mat.vol_pot, Jb, dUj, d2Uj);
+    const double d = A.cB * (kap * d2Ua / W * (SJb - thb * W) + kap * dUb - Pb);
+    const double I6[6] = {1, 1, 1, 0, 0, 0};
+    QpTangent tg;
+    spatial_update<false>(A.mat, Fb, Jb, I6, 0.0, tg, nullptr, nullptr);
+    const double dp = Pb * Jb - kap * Jb * dUj, cw = A.cB * w, dw = d * w * Ja;
+    double T[6];
+#pragma unroll
+    for (int v = 0; v < 6; v++) T[v] = cw * (tg.tau[v] + (v < 3 ? dp : 0.0));
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      double ga[3], gb[3], y[3];
+#pragma unroll
+      for (int j = 0; j < 3; j++) {
+        ga[j] = dXi[c * 3] * Fia[j] + dXi[c * 3 + 1] * Fia[3 + j] + dXi[c * 3 + 2] * Fia[6 + j];
+        gb[j] = dXi[c * 3] * Fib[j] + dXi[c * 3 + 1] * Fib[3 + j] + dXi[c * 3 + 2] * Fib[6 + j];
+      }
+      smv(T, gb, y);
+#pragma unroll
+      for (int i = 0; i < 3; i++) M[i * 3 + c] = fma(dw, ga[i], y[i]);
+    }
+  }
+#pragma unroll
+  for (int b = 0; b < 10; b++)
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+      out[3 * b + i] = M[i * 3] * sdN[q][b][0] + M[i * 3 + 1] * sdN[q][b][1] + M[i * 3 + 2] * sdN[q][b][2] - sN[q][b] * f[i];
+  // lane q ends with the sums of values 8 q .. 8 q + 7
+#pragma unroll
+  for (int i = 0; i < 16; i++) {
+    const double give = (q & 2) ? out[i] : out[16 + i], keep = (q & 2) ? out[16 + i] : out[i];
+    out[i] = keep + __shfl_xor_sync(FULL, give, 2);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const double give = (q & 1) ? out[i] : out[8 + i], keep = (q & 1) ? out[8 + i] : out[i];
+    out[i] = keep + __shfl_xor_sync(FULL, give, 1);
+  }
+  if (!in) return;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int k = 8 * q + i;
+    if (k >= 30) continue;
+    const int b = k / 3, c = k - 3 * b;
+    const int id = A.dof[c * A.nn + A.conn[(long)b * A.ne + e]];
+    if (id > 0) atomicAdd(A.R + (id - 1), out[i]);
   }
 }
 

@@ -124,8 +124,8 @@ struct pgfem_gpu_ctx {
   double *tr_buf = nullptr;
   double *tr_F = nullptr;  // crystal plasticity: F at t_n and t_{n-1} per element (SoA 2 x 9*ne)
   // three-field transient: P_n, theta_n, P_{n-1}, theta_{n-1} per element
-  // (4*ne), and scratch for the mid-point P, theta (4*ne) and u_{n-1+a} at
-  // the nodes (3*nn)
+  // (4*ne), and scratch for the mid-point P, theta (4*ne), u_{n-1+a} and
+  // the inertia combination at the nodes (3*nn each)
   double *tf_hist = nullptr, *tf_mid = nullptr;
   // transient calls: minus the consistent mass of unit density, CSR-aligned
   // (nnz; geometry only, formed on the first transient R+K call)
@@ -379,6 +379,7 @@ AsmArgs base_args(const pgfem_gpu_ctx *c) {
   a.elem_group = c->elem_group;
   a.F0_tab = c->F0_tab;
   a.wait_ns = c->wait_ns;
+  a.rscale = 1.0;
   return a;
 }
 
@@ -421,7 +422,7 @@ int launch_asm(const AsmArgs &a, long nitems, cudaStream_t s) {
 // 26-double records for the tensor-core quadratic-tet kernel, 30 for its
 // three-field form, 38 for the linear-tet kernels).
 template <int NNE, int NQP, int MODEL, bool TF = false>
-int launch_qp_update(pgfem_gpu_ctx *c, cudaStream_t s) {
+int launch_qp_update(pgfem_gpu_ctx *c, cudaStream_t s, double wscale = 1.0) {
   constexpr bool YREC = NNE == 10;
   const int nf = YREC ? yrec_fields(TF) : kQRec;
   // the tiled layout of the 10-node records is padded to whole tiles
@@ -455,6 +456,7 @@ int launch_qp_update(pgfem_gpu_ctx *c, cudaStream_t s) {
   q.shp = c->shp;
   q.tf_P = c->tf_P;
   q.tf_theta = c->tf_theta;
+  q.wscale = wscale;
   k_qp_update<NNE, NQP, MODEL, YREC, TF><<<(unsigned)((c->nqp + 127) / 128), 128, 0, s>>>(q);
   CK(cudaGetLastError());
   return PGFEM_GPU_OK;
@@ -463,15 +465,29 @@ int launch_qp_update(pgfem_gpu_ctx *c, cudaStream_t s) {
 // quadratic tets in two kernels: point updates into c->qrec (40-double
 // records; K zeroed meanwhile on the context's second stream), then the
 // tensor-core element assembly from the records
-template <int MODEL, bool TF = false>
-int launch_p2m(pgfem_gpu_ctx *c, const AsmArgs &a0, cudaStream_t s) {
-  if (!TF && c->three_field) return launch_p2m<MODEL, true>(c, a0, s);
+// K's first write of the tensor-core quadratic-tet path, on the side stream: zeros, or
+// k_c times `from` (nnz).
+int fork_K_init(pgfem_gpu_ctx *c, double *K, cudaStream_t s, const double *from = nullptr, double k_c = 0.0) {
   CK(cudaEventRecord(c->zfork, s));
   CK(cudaStreamWaitEvent(c->zstream, c->zfork, 0));
-  CK(cudaMemsetAsync(a0.K, 0, sizeof(double) * c->nnz, c->zstream));
+  if (from) {
+    k_scale_copy<<<(unsigned)std::min<long>((c->nnz + 255) / 256, 148 * 2), 256, 0, c->zstream>>>(K, k_c, from, c->nnz);
+    CK(cudaGetLastError());
+  } else {
+    CK(cudaMemsetAsync(K, 0, sizeof(double) * c->nnz, c->zstream));
+  }
   CK(cudaMemsetAsync(c->p2m_ticket, 0, sizeof(unsigned), c->zstream));
   CK(cudaEventRecord(c->zjoin, c->zstream));
-  if (int r = launch_qp_update<10, 4, MODEL, TF>(c, s)) return r;
+  return PGFEM_GPU_OK;
+}
+
+// wscale: factor of the records' point weights; K_ready: the caller has called fork_K_init.
+template <int MODEL, bool TF = false>
+int launch_p2m(pgfem_gpu_ctx *c, const AsmArgs &a0, cudaStream_t s, double wscale = 1.0, bool K_ready = false) {
+  if (!TF && c->three_field) return launch_p2m<MODEL, true>(c, a0, s, wscale, K_ready);
+  if (!K_ready)
+    if (int r = fork_K_init(c, a0.K, s)) return r;
+  if (int r = launch_qp_update<10, 4, MODEL, TF>(c, s, wscale)) return r;
   CK(cudaStreamWaitEvent(s, c->zjoin, 0));
   AsmArgs a = a0;
   a.qrec = c->qrec;
@@ -2176,7 +2192,7 @@ __global__ void k_tf_mid(long ne, const double *P, const double *th, const doubl
 // correction kernel's arguments.
 static int tf_transient_prep(pgfem_gpu_ctx *c, double alpha, double dt_np1, double dt_n, TfTrArgs &T) {
   int r;
-  if (!c->tf_mid && (r = dalloc(c, &c->tf_mid, (size_t)4 * c->ne + 3 * c->nn))) return r;
+  if (!c->tf_mid && (r = dalloc(c, &c->tf_mid, (size_t)4 * c->ne + 6 * c->nn))) return r;
   T = TfTrArgs{};
   T.A.X = c->X;
   T.A.unode = c->unode;
@@ -2262,6 +2278,97 @@ static int transient_3f(pgfem_gpu_ctx *c, const double *tu2, const double *tu1, 
   return PGFEM_GPU_OK;
 }
 
+// Minus the consistent mass of unit density, CSR-aligned, formed on first use.
+static int ensure_mass(pgfem_gpu_ctx *c, cudaStream_t s) {
+  if (c->mass_csr) return PGFEM_GPU_OK;
+  if (int r = dalloc(c, &c->mass_csr, std::max<long>(1, c->nnz))) return r;
+  CK(cudaMemsetAsync(c->mass_csr, 0, sizeof(double) * c->nnz, s));
+  InertiaArgs im{};
+  im.X = c->X;
+  im.conn = c->conn;
+  im.dof = c->dof;
+  im.rowptr0 = c->rowptr0;
+  im.rowlen = c->rowlen;
+  im.mask = c->mask;
+  im.pos = c->pos;
+  im.nn = c->nn;
+  im.ne = c->ne;
+  im.vnode = c->unode;  // read, not used: no residual
+  im.cK = 1.0;
+  im.K = c->mass_csr;
+  im.shp = c->shp;
+  const unsigned ge = (unsigned)((c->ne + 127) / 128);
+  if (c->nne == 10) k_inertia<10, 4><<<ge, 128, 0, s>>>(im);
+  else k_inertia<4, 1><<<ge, 128, 0, s>>>(im);
+  CK(cudaGetLastError());
+  return PGFEM_GPU_OK;
+}
+
+// The three-field transient R and K without surface loads: K starts from the mass
+// term on the side stream, the newer mid point's records carry the factor kK (its
+// residual rows the factor cA / kK), and one kernel adds the older point's, the
+// condensation's and the inertia terms of R.  Against transient_3f and the passes of
+// transient_core it saves the pass over K (517 us), the older point's records and
+// residual (250 us) and the correction and inertia kernels (578 us) for one kernel of
+// 257 us that runs beside K's start: 3.01 -> 1.94 ms at 384,000 elements.  Surface
+// loads scale with their own times, so they keep transient_3f.
+static int transient_3f_fused(pgfem_gpu_ctx *c, const double *tu2, const double *tu1, const double *tu0,
+                              const double *tp2, const double *tp1, const double *tp0, double alpha, double dt_np1,
+                              double dt_n, double rho, cudaStream_t s) {
+  TfTrArgs T;
+  int r = tf_transient_prep(c, alpha, dt_np1, dt_n, T);
+  if (r || (r = ensure_mass(c, s))) return r;
+  const unsigned ge = (unsigned)((c->ne + 127) / 128);
+  const long n3 = 3 * c->nn;
+  double *ub = c->tf_mid + (size_t)4 * c->ne, *v = ub + n3;
+  CK(cudaMemsetAsync(c->d_R, 0, sizeof(double) * c->ndof, s));
+  if ((r = fork_K_init(c, c->d_K, s, c->mass_csr, rho / dt_np1))) return r;
+  k_tf_mid<<<ge, 128, 0, s>>>(c->ne, c->tf_P, c->tf_theta, c->tf_hist, alpha, c->tf_mid);
+  k_tr_nodes<<<(unsigned)((n3 + 255) / 256), 256, 0, s>>>(c->dof, n3, tu2, tu1, tu0, c->npres ? tp2 : nullptr, tp1, tp0,
+                                                          alpha, dt_np1, dt_n, c->unode, ub, v);
+  TfTrResArgs x{};
+  x.X = c->X;
+  x.ua = c->unode;
+  x.ub = ub;
+  x.v = v;
+  x.conn = c->conn;
+  x.dof = c->dof;
+  x.perm = c->perm;
+  x.nn = c->nn;
+  x.ne = c->ne;
+  x.mid = c->tf_mid;
+  x.R = c->d_R;
+  x.status = c->status;
+  x.mat = c->mat;
+  x.shp = c->shp;
+  x.cB = T.cB;
+  x.cR = rho / (dt_np1 * dt_n);
+  k_tf_transient_terms<<<(unsigned)((4 * c->ne + 127) / 128), 128, 0, s>>>(x);
+  CK(cudaGetLastError());
+  // newer mid point: P_a, theta_a (c->unode holds u_{n+a})
+  double *P_cur = c->tf_P, *th_cur = c->tf_theta;
+  c->tf_P = c->tf_mid;
+  c->tf_theta = c->tf_mid + c->ne;
+  AsmArgs a = base_args(c);
+  a.R = c->d_R;
+  a.K = c->d_K;
+  a.rscale = T.cA / T.kK;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  if (c->timing && c->events.size() < 4096) {
+    CK(cudaEventCreate(&e0));
+    CK(cudaEventCreate(&e1));
+    CK(cudaEventRecord(e0, s));
+  }
+  r = launch_p2m<PGFEM_MODEL_HE, true>(c, a, s, T.kK, true);
+  if (e0) {
+    CK(cudaEventRecord(e1, s));
+    c->events.emplace_back(e0, e1);
+  }
+  c->tf_P = P_cur;
+  c->tf_theta = th_cur;
+  return r;
+}
+
 // The transient element on device buffers (displacements and prescribed
 // values at the three times), into the context's R and K buffers (K when
 // wantK): the surface-load descriptors, the mid-point assemblies and their
@@ -2290,6 +2397,8 @@ static int transient_core(pgfem_gpu_ctx *c, const double *tu2, const double *tu1
     CK(cudaMemcpyAsync(c->nbc_desc_tr, d.data(), sizeof(double) * d.size(), cudaMemcpyHostToDevice, s));
     c->nbc_desc_cur = c->nbc_desc_tr;
   }
+  if (c->three_field && wantK && !c->nbc_nface && uses_p2m(c))
+    return transient_3f_fused(c, tu2, tu1, tu0, tp2, tp1, tp0, alpha, dt_np1, dt_n, rho, s);
   if (c->three_field) {
     r = transient_3f(c, tu2, tu1, tu0, tp2, tp1, tp0, tua, tpa, tR2, alpha, dt_np1, dt_n, wantK, s);
     c->nbc_desc_cur = nullptr;
@@ -2348,16 +2457,7 @@ static int transient_core(pgfem_gpu_ctx *c, const double *tu2, const double *tu1
   if (wantK) {
     // K = kscale K - rho / dt_np1 M: the mid-point stiffness factor (the CP
     // element applies its own) and the consistent mass, in one pass
-    if (!c->mass_csr) {
-      if ((r = dalloc(c, &c->mass_csr, std::max<long>(1, c->nnz)))) return r;
-      CK(cudaMemsetAsync(c->mass_csr, 0, sizeof(double) * c->nnz, s));
-      InertiaArgs im = ia;
-      im.R = nullptr;
-      im.K = c->mass_csr;
-      im.cK = 1.0;
-      if (c->nne == 10) k_inertia<10, 4><<<ge, 128, 0, s>>>(im);
-      else k_inertia<4, 1><<<ge, 128, 0, s>>>(im);
-    }
+    if ((r = ensure_mass(c, s))) return r;
     const double kscale = c->model == PGFEM_MODEL_CP && !c->three_field ? 1.0 : -alpha * (1.0 - alpha) * dt_np1;
     k_scale_add<<<(unsigned)((c->nnz + 255) / 256), 256, 0, s>>>(c->d_K, kscale, c->mass_csr, rho / dt_np1,
                                                                    c->nnz);

@@ -39,6 +39,52 @@ __global__ void k_scale_add(double *y, double a, const double *x, double b, long
   if (i < n) y[i] = x ? a * y[i] + b * x[i] : a * y[i];
 }
 
+// y = a x on few CTAs with four 16-byte loads in flight per thread: it runs beside
+// kernels that need the rest of the SMs' warps (a full grid held them back: 2.12
+// against 1.94 ms for the transient call at 40^3 cells).  y may be the caller's: the
+// 16-byte path only where the alignment allows it.
+__global__ void __launch_bounds__(256, 6) k_scale_copy(double *__restrict__ y, double a, const double *__restrict__ x,
+                                                    long n) {
+  const long nt = (long)gridDim.x * blockDim.x, t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  long done = 0;
+  if (((reinterpret_cast<unsigned long long>(x) | reinterpret_cast<unsigned long long>(y)) & 15) == 0) {
+    const double2 *x2 = reinterpret_cast<const double2 *>(x);
+    double2 *y2 = reinterpret_cast<double2 *>(y);
+    const long rounds = n / (8 * nt);
+#pragma unroll 1
+    for (long r = 0; r < rounds; r++) {
+      const long i = r * 4 * nt + t;
+      double2 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) v[k] = __ldcs(x2 + i + k * nt);
+#pragma unroll
+      for (int k = 0; k < 4; k++) __stcs(y2 + i + k * nt, make_double2(a * v[k].x, a * v[k].y));
+    }
+    done = rounds * 8 * nt;
+  }
+#pragma unroll 1
+  for (long i = done + t; i < n; i += nt) __stcs(y + i, a * __ldcs(x + i));
+}
+
+// The three nodal fields of a transient call from the displacements at t_{n+1},
+// t_n, t_{n-1} (free DOFs and prescribed values): u_{n+a}, u_{n-1+a} and the inertia
+// combination v.
+__global__ void k_tr_nodes(const int *__restrict__ dof, long n3, const double *__restrict__ u2,
+                           const double *__restrict__ u1, const double *__restrict__ u0,
+                           const double *__restrict__ p2, const double *__restrict__ p1,
+                           const double *__restrict__ p0, double a, double dt1, double dt0, double *__restrict__ ua,
+                           double *__restrict__ ub, double *__restrict__ v) {
+  const long n = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (n >= n3) return;
+  const int id = dof[n];
+  double x2 = 0.0, x1 = 0.0, x0 = 0.0;
+  if (id > 0) x2 = u2[id - 1], x1 = u1[id - 1], x0 = u0[id - 1];
+  else if (id < 0 && p2) x2 = p2[-id - 1], x1 = p1[-id - 1], x0 = p0[-id - 1];
+  ua[n] = (1.0 - a) * x1 + a * x2;
+  ub[n] = (1.0 - a) * x0 + a * x1;
+  v[n] = dt0 * x2 + -(dt1 + dt0) * x1 + dt1 * x0;
+}
+
 struct InertiaArgs {
   const double *X;       // 3*nn SoA
   const int *conn;       // NNE*ne
