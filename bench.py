@@ -317,9 +317,9 @@ def run_ours(args, ws, rank, local):
                 "peak_source": hbm_src}
     roof["frac"] = roof["achieved"] / roof["peak"]
     roof["kernel"] = ("k_assemble<4,1,0> (fused R+K)" if he else
-                      "k_qp_update<10,4,0,1,1> + k_assemble_p2m<0,1> (three-field point updates, then the condensed "
-                      "R+K on the FP64 tensor cores)" if tf else
-                      "k_qp_update<10,4,1,1> + k_assemble_p2m<1> (point updates, then R+K on the FP64 tensor cores)")
+                      "k_qp_update<10,4,0,1,1> + k_assemble_p2r<0,1> (three-field point updates, then the condensed "
+                      "R+K, a warp per element)" if tf else
+                      "k_qp_update<10,4,1,1> + k_assemble_p2r<1> (point updates, then R+K, a warp per element)")
     roof["traffic"] = None if (he or tf) else traffic_per_launch()
     roof["kernel_ms"] = k_ms
     roof["roofline_ms"] = 1e3 * max(t_fp64, t_hbm)

@@ -38,7 +38,7 @@ constexpr int kGVal = 31;         // doubles per incidence: three 3x3 blocks and
 __host__ __device__ constexpr int gather_zero(int most) { return (most + 31) / 32 * 32 * kGVal; }
 // record of HE and J2: G 9, V 6, w a2, c, w a4, w a5, h, h + w p_J (p_J the volumetric
 // stress; s'' = c V = -2/3 w s), one pad: the 26 numbers of the quadratic tets'
-// record (assemble_mma.cuh) without T' = (h + w p_J) 1 + w s
+// record (assemble_p2.cuh) without T' = (h + w p_J) 1 + w s
 constexpr int kP1Rec = 22;
 
 // Lists of the row owners (groups), in order of their first row.

@@ -1,7 +1,7 @@
 // assemble_p1.cuh -- FP64 R+K assembly of linear tets (configs 1 and 5) with
 // column-split block rows: the R+K path of 4-node elements for meshes whose row
 // owners' lists cannot be built (assemble_gather.cuh otherwise).  The
-// point updates run first in k_qp_update<4, 1, MODEL> (assemble_mma.cuh: one
+// point updates run first in k_qp_update<4, 1, MODEL> (assemble_p2.cuh: one
 // thread per point, records in HBM); k_assemble_p1ws is a producer/consumer
 // pipeline over tiles of elements.
 //

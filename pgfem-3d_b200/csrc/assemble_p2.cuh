@@ -1,5 +1,5 @@
-// assemble_mma.cuh -- FP64 R+K assembly of quadratic tets with the element
-// contraction on the FP64 tensor cores (mma.sync .m8n8k4 .f64).
+// assemble_p2.cuh -- FP64 R+K assembly of quadratic tets from point records, one
+// warp per element.
 //
 // Same operation as the other assembly kernels (fd_residuals_MP +
 // stiffmat_fd_MP for the constitutive-model element, src/fd_residuals.cc:
@@ -8,8 +8,8 @@
 //  k_qp_update<..., YREC = true>  one thread per quadrature point: F, the
 //      constitutive update (run_integration_algorithm,
 //      src/constitutive_model.cc:1100-1129; state n -> n+1) and a 26-double
-//      point record (structure of arrays) from which the assembly forms the
-//      matrices of the element contraction:
+//      point record from which the assembly forms the matrices of the element
+//      contraction:
 //        G = (dX/dxi)^-1 F^-1      (p_a = G^T dN_a/dxi = F^-T grad_X N_a)
 //        T' = a1 w/2 1 + w tau,  s'' = -2/3 w s,  U' = w a2 1 + s'',
 //        W' = w (a4 n + a5 dev(n^2)),  h = a1 w / 2
@@ -17,32 +17,37 @@
 //      + a4 n(x)n + a5 n(x)dev(n^2) (cm_models.cuh) and w = det(dX/dxi) x weight.
 //      At a plastic point s = |s| n (radial return), so the record holds
 //      V = n and s'' = c V with c = -2/3 w (s : n); elsewhere V = s,
-//      c = -2/3 w and a4 = a5 = 0.
+//      c = -2/3 w and a4 = a5 = 0.  A warp's records are contiguous: staged in
+//      shared memory and written by one bulk copy.
 //
-//  k_assemble_p2m  persistent grid over tiles of 4 consecutive elements, four
-//      warps per CTA, one element per warp in the contraction.  With the
-//      vectors p, T = T'p, U = U'p, W = W'p, h p of node b at point q, the
-//      element block K_ab[i][k] (compute_stiffness_matrix,
-//      src/constitutive_model.cc:1520-1616, in spatial form) is
-//        K_ab[i][k] = sum_q sum_j p_a[j] Y_q[j][(b,i,k)],
-//        Y_q[j][(b,i,k)] = d_jk h p_b[i] + d_ij U_b[k] + s''_ij p_b[k]
-//                          + n_ij W_b[k] + d_ik T_b[j],
-//      and the residual R_a[i] = sum_q sum_j p_a[j] w tau_ij
-//      (compute_residual_vector, :1628-1662): one GEMM per element,
-//        C (96 x 10) = Y^T (96 x 12) P (12 x 10),  P[(q,j)][a] = p_qa[j],
-//      whose 96 rows are (i, b, k) in blocks of 32 per i (30 K columns, the
-//      residual, one pad) and whose 12-deep contraction runs over (q, j).
-//   Y  all threads: item (element, point, column node b) builds its 27 Y
-//      values and its p into shared memory (Y in the A-fragment order of the
-//      mma, so that each fragment load is 32 consecutive doubles), and the
-//      column offsets of node b's block in the rows of the element's nodes;
-//   C  warp per element: 36 mma.m8n8k4 for row nodes a = 0..7 and 36 more on
-//      the same A fragments for row nodes 8 and 9 (B columns p_8, p_9
-//      repeated, so that every lane holds its row tiles' results);
-//   S  FP64 reductions of the 900 K entries and 30 R entries into the CSR
-//      through the node-block map (fd_res_assemble, src/fd_residuals.cc:58-73;
-//      PLoc_Sparse, src/PLoc_Sparse.cc:15-175).  Per reduction instruction a
-//      warp writes eight consecutive entries of four CSR rows.
+//  k_assemble_p2r  persistent grid, one element per warp at a time.  With p of node
+//      b at point q, T = T'p, U = U'p, W = W'p, the element block K_ab[i][k]
+//      (compute_stiffness_matrix, src/constitutive_model.cc:1520-1616, in spatial
+//      form) is
+//        K_ab[i][k] = sum_q sum_j p_a[j] Y_q[j][i],
+//        Y_q[j][i] = d_jk h p_b[i] + d_ij U_b[k] + s''_ij p_b[k] + n_ij W_b[k] + d_ik T_b[j]
+//      for lane (b, k), and lane 30 holds the residual R_a[i] with Y = w tau
+//      (compute_residual_vector, :1628-1662).  A lane builds its Y in registers
+//      and Z_q = G_q Y_q, the derivatives by the corners' barycentric coordinates
+//      (Z of corner 0 = -sum of the others).  dN_a is linear in those, lambda_l(q)
+//      = B + (A - B) d_lq by the rule, so the sum over a point's ten nodes reduces
+//      to S_l = sum_q Z_q,l, the corner's own Z, and one sum per edge: 24 FP64
+//      operations per point and lane where the plain contraction takes 90.
+//      The columns of one row (node a, component i) then are the warp's lanes: one
+//      reduction instruction writes the element's 30 entries of a row, so that
+//      neighbouring column nodes share the 32-byte sectors (340 sectors per
+//      element, against 440 for eight columns of four rows), through the
+//      node-block map (fd_res_assemble, src/fd_residuals.cc:58-73; PLoc_Sparse,
+//      src/PLoc_Sparse.cc:15-175).
+//      What bounds it is the rate of FP64 reductions in L2 (about 300e9 per second
+//      measured, whatever the sectors), so a warp takes runs of up to eight consecutive
+//      elements and hands the entries of two nodes that the next element has too
+//      to that element through shared memory (930 -> about 680 reductions per
+//      element with the face-chained processing order).
+//      Against the earlier kernel (Y through shared memory, the contraction on the
+//      FP64 tensor cores at 96 x 16 x 12 padded, a scatter of eight columns of four
+//      rows): J2, 1.57 M elements, whole call 6003 -> 5224 us; three-field, 146,334
+//      elements, 612 -> 502 us; J2, 2,058 elements, 28.9 -> 26.7 us.
 #pragma once
 #include <cstdint>
 
@@ -52,18 +57,14 @@
 namespace pgb {
 
 constexpr int kQRec = kRec;  // point record of the linear-tet path: G 9, w, tau 6, s 6, n 6, dev(n^2) 6, a1 a2 a4 a5
-// point record of the tensor-core path: G 9, T' 6, V 6, w a2, c, w a4, w a5, h
+// point record of the quadratic-tet path, one point after the other in processing
+// order: T' 6, V 6, G 9, w a2, c, w a4, w a5, h
+constexpr int kYT = 0, kYV = 6, kYG = 12, kYWa2 = 21, kYC = 22, kYW4 = 23, kYW5 = 24, kYH = 25;
 constexpr int kYRec = 26;
 // the three-field (CM3F) element adds w J, w and the element's theta and P
+constexpr int kYWJ = 26, kYW = 27, kYTheta = 28, kYP = 29;
 constexpr int kYRecTF = 30;
 __host__ __device__ constexpr int yrec_fields(bool tf) { return tf ? kYRecTF : kYRec; }
-constexpr int kMPtsT = 16;  // points per record tile (the assembly tile: 4 elements x 4 points)
-
-// index of field c of record slot qs in the tiled layout of the tensor-core path
-template <int NRF = kYRec>
-__host__ __device__ __forceinline__ long yrec_idx(long qs, int c) {
-  return ((qs >> 4) * NRF + c) * kMPtsT + (qs & (kMPtsT - 1));
-}
 
 struct QpArgs {
   const double *X;      // 3*nn
@@ -75,8 +76,7 @@ struct QpArgs {
   const double *F0_tab;   // group -> macro deformation (9)
   const double *state_n;
   double *state_np1;
-  double *qrec;         // kQRec*nqp (SoA) or, for 10-node elements, kYRec doubles per point in
-                        // tiles of kMPtsT points ([tile][field][point], padded to whole tiles)
+  double *qrec;         // kQRec*nqp (SoA) or, for 10-node elements, kYRec (kYRecTF) doubles per point
   unsigned long long *status;
   // processing order: record slot e' holds element perm[e'] (nullptr: e' = e);
   // the state stays in element order
@@ -89,13 +89,13 @@ struct QpArgs {
   double wscale;  // factor of every record's point weight (the transient's factor of K)
 };
 
-template <int NNE, int NQP, int MODEL, bool YREC = false, bool TF = false>
-__global__ void __launch_bounds__(128) k_qp_update(const QpArgs A) {
+// One point: rec is its record (YREC: NRF doubles, 16-byte aligned) or the first
+// field's array (SoA of nqp).
+template <int NNE, int NQP, int MODEL, bool YREC, bool TF>
+__device__ __forceinline__ void qp_point(const QpArgs &A, long qs, double *rec) {
   constexpr bool PLASTIC = (MODEL == 1);
   constexpr int NRF = yrec_fields(TF);
   constexpr int NR = YREC ? NRF : kQRec;
-  const long qs = blockIdx.x * (long)blockDim.x + threadIdx.x;  // record slot
-  if (qs >= A.nqp) return;
   const long es = qs / NQP;
   const int q = (int)(qs - es * NQP);
   const long e = A.perm ? (long)A.perm[es] : es;
@@ -116,7 +116,6 @@ __global__ void __launch_bounds__(128) k_qp_update(const QpArgs A) {
       dU[i * 3 + 2] += g2 * u;
     }
   }
-  double *rec = A.qrec;
   const long S = A.nqp;
   const double detJ = det3(dX);
   double dXi[9], F[9], Fi[9];
@@ -138,7 +137,7 @@ __global__ void __launch_bounds__(128) k_qp_update(const QpArgs A) {
   if (!ok) {
     atomicAdd(&A.status[0], 1ull);
 #pragma unroll
-    for (int c = 0; c < NR; c++) rec[YREC ? yrec_idx<NRF>(qs, c) : c * S + qs] = 0.0;
+    for (int c = 0; c < NR; c++) rec[YREC ? c : c * S + qs] = 0.0;
     return;
   }
   double Ast[6] = {1, 1, 1, 0, 0, 0}, alpha = 0.0;
@@ -169,35 +168,42 @@ __global__ void __launch_bounds__(128) k_qp_update(const QpArgs A) {
     for (int c = 0; c < 6; c++) A.state_np1[c * S + qp] = Anp1[c];
     A.state_np1[6 * S + qp] = alpha_np1;
   }
+  double G[9];
 #pragma unroll
   for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int j = 0; j < 3; j++)
-      rec[YREC ? yrec_idx<NRF>(qs, i * 3 + j) : (i * 3 + j) * S + qs] =
-          dXi[i * 3 + 0] * Fi[0 * 3 + j] + dXi[i * 3 + 1] * Fi[1 * 3 + j] + dXi[i * 3 + 2] * Fi[2 * 3 + j];
+      G[i * 3 + j] = dXi[i * 3 + 0] * Fi[0 * 3 + j] + dXi[i * 3 + 1] * Fi[1 * 3 + j] + dXi[i * 3 + 2] * Fi[2 * 3 + j];
   const double w = detJ * A.shp.w[q] * A.wscale;
   if (YREC) {
     const double h = 0.5 * t.a1 * w, c23 = (2.0 / 3.0) * w;
     // plastic point: n != 0 (the unit flow direction, s = (s : n) n)
     const bool pl = PLASTIC && (t.n[0] != 0.0 || t.n[1] != 0.0 || t.n[2] != 0.0 || t.n[3] != 0.0 ||
                                 t.n[4] != 0.0 || t.n[5] != 0.0);
+    double r[NRF];
 #pragma unroll
     for (int c = 0; c < 6; c++) {
-      rec[yrec_idx<NRF>(qs, 9 + c)] = h * (c < 3 ? 1.0 : 0.0) + w * t.tau[c];
-      rec[yrec_idx<NRF>(qs, 15 + c)] = pl ? t.n[c] : t.s[c];
+      r[kYT + c] = h * (c < 3 ? 1.0 : 0.0) + w * t.tau[c];
+      r[kYV + c] = pl ? t.n[c] : t.s[c];
     }
-    rec[yrec_idx<NRF>(qs, 21)] = w * t.a2;
-    rec[yrec_idx<NRF>(qs, 22)] = pl ? -c23 * sdot(t.s, t.n) : -c23;
-    rec[yrec_idx<NRF>(qs, 23)] = w * t.a4;
-    rec[yrec_idx<NRF>(qs, 24)] = w * t.a5;
-    rec[yrec_idx<NRF>(qs, 25)] = h;
+#pragma unroll
+    for (int c = 0; c < 9; c++) r[kYG + c] = G[c];
+    r[kYWa2] = w * t.a2;
+    r[kYC] = pl ? -c23 * sdot(t.s, t.n) : -c23;
+    r[kYW4] = w * t.a4;
+    r[kYW5] = w * t.a5;
+    r[kYH] = h;
     if (TF) {
-      rec[yrec_idx<NRF>(qs, 26)] = w * J;
-      rec[yrec_idx<NRF>(qs, 27)] = w;
-      rec[yrec_idx<NRF>(qs, 28)] = tfTh;
-      rec[yrec_idx<NRF>(qs, 29)] = tfP;
+      r[kYWJ] = w * J;
+      r[kYW] = w;
+      r[kYTheta] = tfTh;
+      r[kYP] = tfP;
     }
+#pragma unroll
+    for (int c = 0; c < NRF; c += 2) *reinterpret_cast<double2 *>(rec + c) = make_double2(r[c], r[c + 1]);
   } else {
+#pragma unroll
+    for (int c = 0; c < 9; c++) rec[c * S + qs] = G[c];
     rec[9 * S + qs] = w;
 #pragma unroll
     for (int c = 0; c < 6; c++) {
@@ -213,40 +219,59 @@ __global__ void __launch_bounds__(128) k_qp_update(const QpArgs A) {
   }
 }
 
-// ---- tensor-core element assembly ------------------------------------------
-
-constexpr int kMTE = 4;                 // elements per tile (one per warp)
-constexpr int kMThreads = 32 * kMTE;    // 128
-constexpr int kMPts = kMTE * 4;         // points per tile
-// Y doubles per element: [kstep 3][row tile 12][lane 32], and P doubles per
-// element: [a 10][t 12]; both padded so that the item stores of a half-warp
-// (four column-node pairs x four points, possibly of two elements) hit 16
-// distinct banks
-constexpr int kMY = 3 * 12 * 32 + 12;
-constexpr int kMP = 10 * 12 + 4;
-constexpr int kMCS = 36;                // column-table row stride (words): lane loads hit 32 banks
-// column table per element: [a 10][rr = 3 b + k, 30 -> R, 31 -> pad], element stride padded by three
-// words so that the item stores (element, column-node pair, point) spread over the banks
-constexpr int kMCol = 10 * kMCS + 3;
-constexpr int kMMeta = kMTE * 10;       // (element, node) pairs per tile
-constexpr int kMColR = -2;              // column-table marker of the residual row
-// Per-element scatter block (int32 words, 464 bytes so that it copies in 16-byte chunks):
-//   [0, 30)    row base of (node a, component i): CSR offset of the row, -1 if not free
-//   [30, 60)   residual index of (a, i): free DOF id - 1, -1 if not free
-//   [60, 110)  node-pair positions pos[a][b] (uint16, column offset of b's block in a's rows)
-//   [110, 113) free-component masks of the ten nodes (bytes)
-constexpr int kEBW = 116;
-constexpr int kEBPos = 60, kEBMask = 110;
-
-inline size_t p2m_smem_bytes(bool tf = false) {
-  return sizeof(double) * ((size_t)kMTE * kMY + (size_t)kMTE * kMP + (size_t)yrec_fields(tf) * kMPts) +
-         sizeof(int) * (size_t)kMTE * kMCol + sizeof(int) * 2 * (size_t)kMTE * kEBW + 2 * sizeof(uint64_t) +
-         2 * sizeof(long);
+template <int NNE, int NQP, int MODEL, bool YREC = false, bool TF = false>
+__global__ void __launch_bounds__(128) k_qp_update(const QpArgs A) {
+  const long qs = blockIdx.x * (long)blockDim.x + threadIdx.x;  // record slot
+  if (!YREC) {
+    if (qs < A.nqp) qp_point<NNE, NQP, MODEL, YREC, TF>(A, qs, A.qrec);
+    return;
+  }
+  // the warp's records are contiguous: staged in shared memory, written by one bulk copy
+  constexpr int NRF = YREC ? yrec_fields(TF) : 2;
+  __shared__ __align__(16) double stage[4][32 * NRF];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (qs < A.nqp) qp_point<NNE, NQP, MODEL, YREC, TF>(A, qs, stage[warp] + lane * NRF);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  const long q0 = qs - lane;
+  if (lane == 0 && q0 < A.nqp) {
+    const long n = A.nqp - q0 < 32 ? A.nqp - q0 : 32;
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(A.qrec + q0 * NRF),
+                 "r"((unsigned)__cvta_generic_to_shared(stage[warp])), "r"((unsigned)(n * NRF * sizeof(double)))
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
+  }
 }
 
-// bytes of one tile's copies: its point records and its elements' scatter blocks
-__host__ __device__ constexpr unsigned tile_bytes(bool tf) {
-  return (unsigned)(sizeof(double) * yrec_fields(tf) * kMPtsT + sizeof(int) * kMTE * kEBW);
+// ---- element assembly -------------------------------------------------------
+
+constexpr int kP2Threads = 128;
+// Longest run of elements: longer ones hand over more entries, but spread the
+// warps over more of the mesh than L2 holds the rows of (1.57 M elements, call time
+// for 4, 8, 16, 32: 5.72, 5.16, 6.08, 6.72 ms).
+constexpr int kP2Run = 8;
+// Per-element scatter block (int32 words, 480 bytes so that it copies in 16-byte chunks):
+//   [0, 30)    row base of (node a, component i): CSR offset of the row, -1 if not free
+//   [32, 62)   residual index of (a, i): free DOF id - 1, -1 if not free
+//   [64, 114)  node-pair positions pos[a][b] (uint16, column offset of b's block in a's rows)
+//   [114, 117) free-component masks of the ten nodes (bytes)
+//   [117, 119) 4 bits per node: its local number in the previous element of the
+//              processing order, 15 when not there
+//   [119]      bit a: node a is in the next element too
+constexpr int kEBW = 120;
+constexpr int kEBRes = 32, kEBPos = 64, kEBMask = 114, kEBPrev = 117, kEBNext = 119;
+// the four-point rule: point q has barycentric coordinate A at corner (q + 1) mod 4, B at the others
+constexpr double kP2RuleA = 0.58541020, kP2RuleB = 0.13819660;
+
+constexpr int kP2Stage = 30 * 32;  // doubles of the values an element hands to the next one: [row 3 a + i][lane]
+
+// bytes of one element's copies: its point records and its scatter block
+__host__ __device__ constexpr unsigned p2r_elem_bytes(bool tf) {
+  return (unsigned)(4 * sizeof(double) * yrec_fields(tf) + sizeof(int) * kEBW);
+}
+inline size_t p2r_smem_bytes(bool tf) {
+  return (size_t)(kP2Threads / 32) * 2 *
+         (p2r_elem_bytes(tf) + kP2Stage * sizeof(double) + sizeof(uint64_t));
 }
 
 // one-dimensional bulk copy global -> shared through the tensor memory
@@ -276,337 +301,272 @@ __global__ void k_build_eblock(const int *conn, long ne, const int *dof, long nn
   int *o = eb + es * kEBW;
   uint16_t *o16 = reinterpret_cast<uint16_t *>(o + kEBPos);
   uint8_t *o8 = reinterpret_cast<uint8_t *>(o + kEBMask);
+  const long ep = es > 0 ? (perm ? (long)perm[es - 1] : es - 1) : -1;
+  const long en = es + 1 < ne ? (perm ? (long)perm[es + 1] : es + 1) : -1;
+  unsigned long long prev = 0;
+  int next = 0;
   for (int a = 0; a < 10; a++) {
     const int n = conn[(long)a * ne + e];
     const unsigned mk = mask[n];
+    unsigned long long pa = 15;
+    for (int x = 0; x < 10; x++) {
+      if (ep >= 0 && conn[(long)x * ne + ep] == n) pa = x;
+      if (en >= 0 && conn[(long)x * ne + en] == n) next |= 1 << a;
+    }
+    prev |= pa << (4 * a);
     for (int i = 0; i < 3; i++) {
       const bool fr = (mk >> i) & 1u;
       o[a * 3 + i] = fr ? rowptr0[n] + __popc(mk & ((1u << i) - 1u)) * rowlen[n] : -1;
-      o[30 + a * 3 + i] = fr ? dof[i * nn + n] - 1 : -1;
+      o[kEBRes + a * 3 + i] = fr ? dof[i * nn + n] - 1 : -1;
     }
     for (int b = 0; b < 10; b++) o16[a * 10 + b] = pos[(e * 10 + a) * 10 + b];
     o8[a] = (uint8_t)mk;
   }
   o8[10] = o8[11] = 0;
-  o[113] = o[114] = o[115] = 0;
+  o[30] = o[31] = o[62] = o[63] = -1;
+  o[kEBPrev] = (int)(prev & 0xffffffffull);
+  o[kEBPrev + 1] = (int)(prev >> 32);
+  o[kEBNext] = next;
 }
 
-// index of Y[t][r] (t = 3q + j, r = 32 i + 3 b + k) in the fragment-ordered buffer
-__device__ __forceinline__ int y_idx(int t, int r) {
-  return (((t >> 2) * 12 + (r >> 3)) << 5) + ((r & 7) << 2) + (t & 3);
+// predicated shared accesses and reduction, without branches around them
+__device__ __forceinline__ double lds_if(unsigned a, bool on) {
+  double v;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t@q ld.shared.f64 %0, [%1];\n\t}"
+               : "=d"(v)
+               : "r"(a), "r"((unsigned)on)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts_if(unsigned a, double v, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.shared.f64 [%0], %1;\n\t}" ::"r"(a), "d"(v),
+               "r"((unsigned)on)
+               : "memory");
+}
+__device__ __forceinline__ void red_if(double *p, double v, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q red.relaxed.gpu.global.add.f64 [%0], %1;\n\t}" ::"l"(p),
+               "d"(v), "r"((unsigned)on)
+               : "memory");
 }
 
-// D (8x8) += A (8x4, row) B (4x8, col), FP64.  Lane l holds A[l/4][l%4],
-// B[l%4][l/4], and C[l/4][2 (l%4) + c] in c<c>.
-__device__ __forceinline__ void dmma884(double &c0, double &c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
+// edge node (less four) between two corners: 01 12 02 03 13 23
+__host__ __device__ __forceinline__ constexpr int p2_edge(int c, int d) {
+  const int lo = c < d ? c : d, hi = c < d ? d : c;
+  return lo == 0 ? (hi == 1 ? 0 : hi) : lo == 1 ? (hi == 2 ? 1 : 4) : 5;
 }
 
-
-// Item (point q, column nodes b0 and b0 + 5) of one element: p_b into P, the
-// 27 values Y_q[j][(b, i, k)] of each column node and, for b0 = 0, the
-// residual rows Y_q[j][32 i + 30] = w tau_ij (times rscale, the transient's ratio of
-// the residual's factor to the stiffness's, which the records carry).  rec: the point's record fields
-// with stride RS (the element's other points at rec - q + q'); shp: the
-// shape-function derivatives.
-// TF (three-field element, one pressure P and one volume theta per element):
-// the static condensation of (P, theta) adds c Kup Kup^T to the element's K and
-// s Kup to its R, with Kup_b = sum_q w J p_qb (the derivative of the volume
-// constraint), W = sum_q w, fp = sum_q w J - theta W, c = kappa U''(theta) / W
-// and s = c fp + kappa U'(theta) - P -- in the contraction, w J c Kup_b[k] is
-// added to U_b[k] and w J s delta_ij to the residual rows (the pressure part
-// of the point's stress is P J 1 already, from the point kernel).
-// Y[t][r] sits at y_idx(t, r) = tb(t) + 128 i + gk(3 b + k) for r = 32 i + 3 b + k.
-template <bool PLASTIC, int RS, bool TF = false>
-__device__ __forceinline__ void p2m_item(const double *rec, const ShapeTable &shp, int q, int b0, double *Y,
-                                         double *P, const Mat &mat, double rscale) {
-  const double(*dN)[3] = shp.dNxi[q];
-  double G[9], Tm[6], Um[6], Wm[6], s2[6], nn[6];
-#pragma unroll
-  for (int c = 0; c < 9; c++) G[c] = rec[c * RS];
-  const double wa2 = rec[21 * RS], cs = rec[22 * RS], h = rec[25 * RS];
-#pragma unroll
-  for (int c = 0; c < 6; c++) {
-    Tm[c] = rec[(9 + c) * RS];
-    nn[c] = rec[(15 + c) * RS];
-    s2[c] = cs * nn[c];
-    Um[c] = s2[c] + (c < 3 ? wa2 : 0.0);
-  }
-  if (PLASTIC) {
-    // W' = w a4 n + w a5 dev(n^2) (zero at elastic points: w a4 = w a5 = 0)
-    const double w4 = rec[23 * RS], w5 = rec[24 * RS];
-    const double *n = nn;
-    double n2[6];
-    n2[0] = n[0] * n[0] + n[5] * n[5] + n[4] * n[4];
-    n2[1] = n[5] * n[5] + n[1] * n[1] + n[3] * n[3];
-    n2[2] = n[4] * n[4] + n[3] * n[3] + n[2] * n[2];
-    n2[3] = n[5] * n[4] + n[1] * n[3] + n[3] * n[2];
-    n2[4] = n[0] * n[4] + n[5] * n[3] + n[4] * n[2];
-    n2[5] = n[0] * n[5] + n[5] * n[1] + n[4] * n[3];
-    const double t3 = (n2[0] + n2[1] + n2[2]) * (1.0 / 3.0);
-#pragma unroll
-    for (int c = 0; c < 6; c++) Wm[c] = w4 * n[c] + w5 * (n2[c] - (c < 3 ? t3 : 0.0));
-  } else {
-#pragma unroll
-    for (int c = 0; c < 6; c++) Wm[c] = nn[c] = 0.0;
-  }
-  double wJq = 0.0, tfc = 0.0, tfs = 0.0;
-  if (TF) {
-    const double *r0 = rec - q;  // point 0 of the element
-    double W = 0.0, SJ = 0.0;
-#pragma unroll
-    for (int qq = 0; qq < 4; qq++) {
-      SJ += r0[26 * RS + qq];
-      W += r0[27 * RS + qq];
-    }
-    wJq = rec[26 * RS];
-    const double th = rec[28 * RS], Pe = rec[29 * RS];
-    double dU, d2U;
-    vol_derivs(mat.vol_pot, th, dU, d2U);
-    tfc = mat.kappa * d2U / W;
-    tfs = tfc * (SJ - th * W) + mat.kappa * dU - Pe;
-  }
-  int tb[3];
-#pragma unroll
-  for (int j = 0; j < 3; j++) {
-    const int t = 3 * q + j;
-    tb[j] = (t >> 2) * 384 + (t & 3);
-  }
-  // full 3x3 index of a Voigt-stored symmetric matrix (xx yy zz yz xz xy)
-  auto vo = [](int i, int j) { return i == j ? i : 6 - i - j; };
-#pragma unroll
-  for (int half = 0; half < 2; half++) {
-    const int b = b0 + 5 * half;
-    const double g0 = dN[b][0], g1 = dN[b][1], g2 = dN[b][2];
-    double p[3], T[3], U[3], W[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-    for (int j = 0; j < 3; j++) p[j] = G[j] * g0 + G[3 + j] * g1 + G[6 + j] * g2;
-    smv(Tm, p, T);
-    smv(Um, p, U);
-    if (PLASTIC) smv(Wm, p, W);
-    if (TF) {
-      // Kup_b = sum over the element's points of w J G^T dN_b
-      const double *r0 = rec - q;
-      double v[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-      for (int qq = 0; qq < 4; qq++) {
-        const double *rq = r0 + qq;
-        const double d0 = shp.dNxi[qq][b][0], d1 = shp.dNxi[qq][b][1], d2 = shp.dNxi[qq][b][2];
-        const double wj = rq[26 * RS];
-#pragma unroll
-        for (int j = 0; j < 3; j++) v[j] = fma(wj, rq[j * RS] * d0 + rq[(3 + j) * RS] * d1 + rq[(6 + j) * RS] * d2, v[j]);
-      }
-#pragma unroll
-      for (int k = 0; k < 3; k++) U[k] = fma(wJq * tfc, v[k], U[k]);
-    }
-    int gk[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      const int x = 3 * b + k;
-      gk[k] = ((x >> 3) << 5) + ((x & 7) << 2);
-    }
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        double *Yjk = Y + tb[j] + gk[k];
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-          double y = s2[vo(i, j)] * p[k];
-          if (PLASTIC) y = fma(nn[vo(i, j)], W[k], y);
-          if (j == k) y = fma(h, p[i], y);
-          if (i == j) y += U[k];
-          if (i == k) y += T[j];
-          Yjk[128 * i] = y;
-        }
-      }
-      P[b * 12 + 3 * q + j] = p[j];
-    }
-  }
-  if (b0 == 0) {
-    // w tau = T' - h 1 (row r = 32 i + 30: offset 128 i + 120)
-#pragma unroll
-    for (int j = 0; j < 3; j++)
-#pragma unroll
-      for (int i = 0; i < 3; i++) Y[tb[j] + 128 * i + 120] = rscale * (Tm[vo(i, j)] - (i == j ? h - wJq * tfs : 0.0));
-  }
-}
-
+// Three CTAs per SM, 168 registers (16 spilled words): two CTAs without spills
+// measured 15 % slower at 82,944 elements, four with more spills 8 % slower than two.
 template <int MODEL, bool TF = false>
-__global__ void __launch_bounds__(kMThreads, 4) k_assemble_p2m(const AsmArgs args) {
-  constexpr int NNE = 10, NQP = 4, TE = kMTE, NT = kMThreads;
+__global__ void __launch_bounds__(kP2Threads, 3) k_assemble_p2r(const AsmArgs args, int run) {
   constexpr bool PLASTIC = (MODEL == 1);
   constexpr int NRF = yrec_fields(TF);
-  extern __shared__ __align__(16) double msm[];
-  double *sY = msm;                                          // [TE][kMY]
-  double *sP = sY + TE * kMY;                                // [TE][kMP]
-  double *sRec = sP + TE * kMP;                              // [NRF][kMPts]
-  int *sCol = reinterpret_cast<int *>(sRec + NRF * kMPts);    // [TE][10][kMCS]
-  int *sEB = sCol + TE * kMCol;                              // [2][TE][kEBW]
-  uint64_t *mbar = reinterpret_cast<uint64_t *>(sEB + 2 * TE * kEBW);  // [2]: tile copies landed
-  long *sTile = reinterpret_cast<long *>(mbar + 2);                    // [2]: the tile of each buffer
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr unsigned FULL = 0xffffffffu;
+  extern __shared__ __align__(16) unsigned char p2sm[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr unsigned kElem = p2r_elem_bytes(TF), kRecB = 4u * NRF * (unsigned)sizeof(double);
+  constexpr int NW = kP2Threads / 32;
+  unsigned char *wb = p2sm + (size_t)warp * 2 * kElem;
+  double *stage = reinterpret_cast<double *>(p2sm + (size_t)NW * 2 * kElem) + (size_t)warp * 2 * kP2Stage;
+  uint64_t *mbar = reinterpret_cast<uint64_t *>(p2sm + (size_t)NW * 2 *
+                                                           (kElem + kP2Stage * sizeof(double))) +
+                   2 * warp;
   const long ne = args.ne;
-  const long ntiles = (ne + TE - 1) / TE;
-  // pad rows r = 32 i + 31 of Y stay zero; the column table marks the
-  // residual row (rr = 30) and the pad row (rr = 31)
-  for (int x = tid; x < TE * 12; x += NT) {
-    const int el = x / 12, t = x - el * 12;
+  // lane (b, k): column k of node b in the element's rows; lane 30: the residual
+  const bool isK = lane < 30, isR = lane == 30;
+  const int b = isK ? lane / 3 : 0, k = isK ? lane - 3 * b : 0;
+  double dn[4][3], e[3];
 #pragma unroll
-    for (int i = 0; i < 3; i++) sY[el * kMY + y_idx(t, 32 * i + 31)] = 0.0;
-  }
-  for (int x = tid; x < TE * 10; x += NT) {
-    int *row = sCol + (x / 10) * kMCol + (x % 10) * kMCS;
-    row[30] = kMColR;
-    row[31] = -1;
-  }
-
-  // one tile's point records (5120 contiguous bytes of the tiled layout) and
-  // its elements' scatter blocks (1856 contiguous bytes) by two bulk copies of
-  // the tensor memory accelerator, completing on mbar[buf]; the buffers are
-  // padded to whole tiles, so a partial last tile copies whole too
-  if (tid == 0) {
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) dn[q][c] = isK ? args.shp.dNxi[q][b][c] : 0.0;
+#pragma unroll
+  for (int c = 0; c < 3; c++) e[c] = c == k ? 1.0 : 0.0;
+  auto pick = [&](double x0, double x1, double x2) { return k == 0 ? x0 : (k == 1 ? x1 : x2); };
+  double *const out = isR ? args.R : args.K;
+  if (lane == 0) {
     w_mb_init(&mbar[0], 1);
     w_mb_init(&mbar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  __syncthreads();
-  // Tiles are claimed in order from a global counter (zeroed before the
-  // launch), one tile ahead: all CTAs then work on neighbouring tiles of the
-  // processing order, and the CSR rows they reduce into stay in L2 between
-  // the contributions of neighbouring elements.  Thread 0 claims, records the
-  // tile in sTile[buf] and issues its copies; with no tile left it completes
-  // the buffer's phase by a plain arrive.
-  auto claim = [&](int buf) {  // thread 0
-    const long t = (long)atomicAdd(args.ticket, 1u);
-    sTile[buf] = t;
-    if (t < ntiles) {
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // after the generic reads of the buffers
-      mb_expect_tx(&mbar[buf], tile_bytes(TF));
-      bulk_g2s(sRec, args.qrec + t * (long)(NRF * kMPtsT), sizeof(double) * NRF * kMPtsT, &mbar[buf]);
-      bulk_g2s(sEB + buf * TE * kEBW, args.eblk + t * TE * kEBW, sizeof(int) * TE * kEBW, &mbar[buf]);
-    } else {
-      w_mb_arrive(&mbar[buf]);
-    }
+  __syncwarp();
+  auto load = [&](int buf, long el) {  // lane 0: the copies of element slot el
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // after the generic reads of the buffer
+    unsigned char *dst = wb + (size_t)buf * kElem;
+    mb_expect_tx(&mbar[buf], kElem);
+    bulk_g2s(dst, args.qrec + el * (4 * NRF), kRecB, &mbar[buf]);
+    bulk_g2s(dst + kRecB, args.eblk + el * kEBW, kElem - kRecB, &mbar[buf]);
   };
-  if (tid == 0) claim(0);
-
-  for (int it = 0;; it++) {
-    const int mb = it & 1;
-    // this tile's copies landed (bounded wait: a wait that runs out is
-    // counted in status[3] and every thread leaves, after waiting -- again
-    // bounded -- for the copies still in flight)
-    const bool landed = w_mb_wait(&mbar[mb], (unsigned)((it >> 1) & 1), args.wait_ns);
-    if (__syncthreads_or(!landed)) {  // also: previous tile's C/S done
-      if (tid == 0) {
+  // Runs of `run` elements: one per warp when that covers the mesh, else claimed in
+  // order from one counter (zeroed before the launch; a claim takes about 7 ns of it), so that all warps work on
+  // neighbouring elements of the processing order and the CSR rows they reduce
+  // into stay in L2 between neighbouring elements' contributions.
+  const bool claims = (long)gridDim.x * NW * run < ne;
+  long el = ((long)blockIdx.x * NW + warp) * run, next = ne;  // next: lane 0's claim
+  if (claims) {
+    if (lane == 0) el = (long)atomicAdd(args.ticket, 1u) * run;
+    el = __shfl_sync(FULL, el, 0);
+  }
+  if (lane == 0 && el < ne) load(0, el);
+  for (int it = 0, x = 0; el < ne; it++) {
+    const int buf = it & 1;
+    // bounded wait; one that runs out is counted in status[3] and the warp leaves,
+    // after waiting -- again bounded -- for the copies in flight
+    const bool landed = w_mb_wait(&mbar[buf], (unsigned)((it >> 1) & 1), args.wait_ns);
+    if (!__all_sync(FULL, landed)) {
+      if (lane == 0) {
         atomicAdd(&args.status[3], 1ull);
-        w_mb_wait(&mbar[mb], (unsigned)((it >> 1) & 1), args.wait_ns);
+        w_mb_wait(&mbar[buf], (unsigned)((it >> 1) & 1), args.wait_ns);
       }
       break;
     }
-    const long e0 = sTile[mb] * TE;  // written before the barrier above
-    if (e0 >= ne) break;
-    // ---- Y: items (element, column-node pair, point), point fastest ----
-    if (tid < TE * 20) {
-      const int el = tid / 20, rem = tid - el * 20;
-      const int bp = rem >> 2, q = rem & 3;
-      if (e0 + el < ne) {
-        p2m_item<PLASTIC, kMPts, TF>(sRec + el * NQP + q, args.shp, q, bp, sY + el * kMY, sP + el * kMP,
-                                     args.mat, args.rscale);
-        // column offsets of node b's block inside the rows of nodes a = q, q+4, q+8
-        const int *eb = sEB + (mb * TE + el) * kEBW;
-        const uint16_t *pos16 = reinterpret_cast<const uint16_t *>(eb + kEBPos);
-        const uint8_t *mk8 = reinterpret_cast<const uint8_t *>(eb + kEBMask);
-#pragma unroll
-        for (int half = 0; half < 2; half++) {
-          const int b = bp + 5 * half;
-          const unsigned maskB = mk8[b];
-          int *ct = sCol + el * kMCol + 3 * b;
-#pragma unroll
-          for (int x4 = 0; x4 < 3; x4++) {
-            const int a = q + 4 * x4;
-            if (a < NNE) {
-              const int pab = pos16[a * 10 + b];
-#pragma unroll
-              for (int k = 0; k < 3; k++)
-                ct[a * kMCS + k] = ((maskB >> k) & 1u) ? pab + rank_of(maskB, k) : -1;
-            }
-          }
-        }
-      }
-    }
-    __syncthreads();  // Y, P and column offsets complete; the record buffer is free
-    // ---- claim the next tile, prefetch its records and scatter blocks ----
-    if (tid == 0) claim(mb ^ 1);
-    // ---- C: the element's GEMM on the FP64 tensor cores ----
-    // m8n8k4 for row nodes a = 0..7 (12 row tiles of 8 Y rows, 3 steps over
-    // the contraction) and, on the same A fragments, for row nodes 8 and 9
-    // with B columns (p_8, p_9) repeated four times: lane (rho, u) then holds
-    // C[8 m + rho][8 + c] of every row tile m in a89[m][c], and no lane
-    // exchange is needed to spread rows 8, 9 over the warp for the scatter
-    const int el = warp;
-    if (e0 + el >= ne) continue;
-    const double *Y = sY + el * kMY;
-    const double *P = sP + el * kMP;
-    const int rho = lane >> 2, u = lane & 3;
-    double acc[12][2], a89[12][2];
-#pragma unroll
-    for (int m = 0; m < 12; m++) acc[m][0] = acc[m][1] = a89[m][0] = a89[m][1] = 0.0;
-#pragma unroll
-    for (int s = 0; s < 3; s++) {
-      const double bf = P[rho * 12 + 4 * s + u];
-      const double b89 = P[(8 + (rho & 1)) * 12 + 4 * s + u];
-#pragma unroll
-      for (int m = 0; m < 12; m++) {
-        const double af = Y[(s * 12 + m) * 32 + lane];
-        dmma884(acc[m][0], acc[m][1], af, bf);
-        dmma884(a89[m][0], a89[m][1], af, b89);
-      }
-    }
-    // ---- S: reductions into the CSR ----
-    // C[r][a], r = 8 m + rho = 32 i + rr: K entry (row i of node a, column rr
-    // of the column table) or, for rr = 30, the residual of (a, i); one
-    // reduction instruction per value, its target selected.
-    const int *eb = sEB + (mb * TE + el) * kEBW;
-    const int *ct = sCol + el * kMCol;
-    // the target of value v: K entry (row base rb, column offset cv >= 0) or,
-    // for the residual row (cv = kMColR), the residual entry rd; nothing when
-    // component i of node a is not free (rb < 0) or the column is (cv = -1)
-    auto red = [&](int rb, int rd, int cv, double v) {
-      const bool kk = cv >= 0;
-      if (rb >= 0 && (kk || cv == kMColR)) atomicAdd(kk ? args.K + (rb + cv) : args.R + rd, v);
-    };
-#pragma unroll
-    for (int c = 0; c < 2; c++) {
-      const int a = 2 * u + c;
-      int rb[3], rd[3], cv[4];
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        rb[i] = eb[a * 3 + i];
-        rd[i] = eb[30 + a * 3 + i];
-      }
-#pragma unroll
-      for (int mq = 0; mq < 4; mq++) cv[mq] = ct[a * kMCS + 8 * mq + rho];
-#pragma unroll
-      for (int m = 0; m < 12; m++) red(rb[m >> 2], rd[m >> 2], cv[m & 3], acc[m][c]);
+    const bool more = x + 1 < run && el + 1 < ne;  // this run goes on
+    if (lane == 0) {
+      if (x == 0 && claims) next = (long)atomicAdd(args.ticket, 1u) * run;
+      if (more) load(buf ^ 1, el + 1);
     }
     {
-      // lane u of a row group takes the row tile m = 4 mm + u (row i = mm)
-      const int rr = 8 * u + rho;
-      const int cv8 = ct[8 * kMCS + rr], cv9 = ct[9 * kMCS + rr];
+      const double *rec = reinterpret_cast<const double *>(wb + (size_t)buf * kElem);
+      const int *eb = reinterpret_cast<const int *>(wb + (size_t)buf * kElem + kRecB);
+      double tfc = 0.0, tfs = 0.0, vk = 0.0;
+      if (TF) {
+        double W = 0.0, SJ = 0.0;
 #pragma unroll
-      for (int mm = 0; mm < 3; mm++) {
-        double v8 = a89[4 * mm][0], v9 = a89[4 * mm][1];
-#pragma unroll
-        for (int x = 1; x < 4; x++) {
-          v8 = u == x ? a89[4 * mm + x][0] : v8;
-          v9 = u == x ? a89[4 * mm + x][1] : v9;
+        for (int q = 0; q < 4; q++) {
+          const double *r = rec + q * NRF;
+          const double wJ = r[kYWJ];
+          SJ += wJ;
+          W += r[kYW];
+          vk = fma(wJ, r[kYG + k] * dn[q][0] + r[kYG + 3 + k] * dn[q][1] + r[kYG + 6 + k] * dn[q][2], vk);
         }
-        red(eb[24 + mm], eb[54 + mm], cv8, v8);
-        red(eb[27 + mm], eb[57 + mm], cv9, v9);
+        const double th = rec[kYTheta], Pe = rec[kYP];
+        double dU, d2U;
+        vol_derivs(args.mat.vol_pot, th, dU, d2U);
+        tfc = args.mat.kappa * d2U / W;
+        tfs = tfc * (SJ - th * W) + args.mat.kappa * dU - Pe;
+        vk *= tfc;
       }
+      double S[3][3], C[4][3], E[6][3];
+#pragma unroll
+      for (int l = 0; l < 3; l++)
+#pragma unroll
+        for (int i = 0; i < 3; i++) S[l][i] = 0.0;
+#pragma unroll
+      for (int l = 0; l < 6; l++)
+#pragma unroll
+        for (int i = 0; i < 3; i++) E[l][i] = 0.0;
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const double2 *r2 = reinterpret_cast<const double2 *>(rec + q * NRF);
+        const double2 *v2 = r2 + (isR ? kYT / 2 : kYV / 2);
+        double Tm[6], V[6], G[10];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const double2 t = r2[kYT / 2 + c], v = v2[c];
+          Tm[2 * c] = t.x, Tm[2 * c + 1] = t.y, V[2 * c] = v.x, V[2 * c + 1] = v.y;
+        }
+#pragma unroll
+        for (int c = 0; c < 5; c++) {
+          const double2 g = r2[kYG / 2 + c];
+          G[2 * c] = g.x, G[2 * c + 1] = g.y;
+        }
+        const double2 c4 = r2[kYC / 2], c5h = r2[kYW5 / 2];
+        double p[3], np[3], T[3];
+#pragma unroll
+        for (int j = 0; j < 3; j++) p[j] = G[j] * dn[q][0] + G[3 + j] * dn[q][1] + G[6 + j] * dn[q][2];
+        smv(V, p, np);
+        smv(Tm, p, T);
+        const double pk = pick(p[0], p[1], p[2]), npk = pick(np[0], np[1], np[2]);
+        double U = G[9] * pk + c4.x * npk, m = c4.x * pk;
+        if (PLASTIC) {
+          // (w a4 n + w a5 dev(n^2)) p, n a unit tensor (zero weights at elastic points)
+          const double nnp = pick(V[0], V[5], V[4]) * np[0] + pick(V[5], V[1], V[3]) * np[1] +
+                             pick(V[4], V[3], V[2]) * np[2];
+          m += c4.y * npk + c5h.x * (nnp - (1.0 / 3.0) * pk);
+        }
+        const double wJ = TF ? rec[q * NRF + kYWJ] : 0.0;
+        if (TF) U = fma(wJ, vk, U);
+        m = isR ? args.rscale : m;
+        U = isR ? -args.rscale * (TF ? c5h.y - wJ * tfs : c5h.y) : U;
+        double Y[3][3];
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+          const double hej = c5h.y * e[j];
+#pragma unroll
+          for (int i = 0; i < 3; i++) {
+            double y = fma(e[i], T[j], i == j ? fma(V[i], m, U) : V[6 - i - j] * m);
+            Y[j][i] = fma(hej, p[i], y);
+          }
+        }
+        double Z[4][3];  // by corner
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+#pragma unroll
+          for (int l = 0; l < 3; l++) {
+            Z[l + 1][i] = G[3 * l] * Y[0][i] + G[3 * l + 1] * Y[1][i] + G[3 * l + 2] * Y[2][i];
+            S[l][i] += Z[l + 1][i];
+          }
+          Z[0][i] = -(Z[1][i] + Z[2][i] + Z[3][i]);
+          // edges 01 12 02 03 13 23
+          const int cq = (q + 1) & 3;
+          C[cq][i] = Z[cq][i];
+#pragma unroll
+          for (int o = 0; o < 4; o++)
+            if (o != cq) E[p2_edge(o, cq)][i] += Z[o][i];
+        }
+      }
+      // ---- rows: node a's three rows, 30 consecutive columns of the element per reduction ----
+      constexpr double kC = 4.0 * kP2RuleB - 1.0, kE = 4.0 * kP2RuleB, kG = 4.0 * (kP2RuleA - kP2RuleB);
+      const int *rows = eb + (isR ? kEBRes : 0);
+      const uint16_t *pos16 = reinterpret_cast<const uint16_t *>(eb + kEBPos);
+      const unsigned maskB = reinterpret_cast<const uint8_t *>(eb + kEBMask)[b];
+      const bool live = isR || (isK && ((maskB >> k) & 1u));
+      const int rank = isR ? 0 : rank_of(maskB, k);
+      double S0[3];
+#pragma unroll
+      for (int i = 0; i < 3; i++) S0[i] = -(S[0][i] + S[1][i] + S[2][i]);
+      auto SS = [&](int l, int i) { return l == 0 ? S0[i] : S[l - 1][i]; };
+      int rw[32];
+#pragma unroll
+      for (int c = 0; c < 8; c++) {
+        const int4 v = reinterpret_cast<const int4 *>(rows)[c];
+        rw[4 * c] = v.x, rw[4 * c + 1] = v.y, rw[4 * c + 2] = v.z, rw[4 * c + 3] = v.w;
+      }
+      // entries of two nodes that the next element of the run has too are handed to
+      // it, not reduced
+      const unsigned long long prev = (unsigned)eb[kEBPrev] | (unsigned long long)(unsigned)eb[kEBPrev + 1] << 32;
+      const unsigned nextm = more ? (unsigned)eb[kEBNext] : 0u;
+      const int pb = (int)(prev >> (4 * b)) & 15;
+      const bool take = x > 0 && live && (isR || pb < 10), hand = isR || ((nextm >> b) & 1u);
+      const unsigned st0 = (unsigned)__cvta_generic_to_shared(stage);
+      const unsigned sin = st0 + 8u * (((x + 1) & 1) * kP2Stage + (isR ? lane : 3 * pb + k));
+      const unsigned sout = st0 + 8u * ((x & 1) * kP2Stage + lane);
+      constexpr int el0[6] = {0, 1, 0, 0, 1, 2}, el1[6] = {1, 2, 2, 3, 3, 3};
+#pragma unroll
+      for (int a = 0; a < 10; a++) {
+        const int col = isR ? 0 : (int)pos16[a * 10 + b] + rank;
+        const int pa = (int)(prev >> (4 * a)) & 15;
+        const bool ta = take && pa < 10, ha = hand && ((nextm >> a) & 1u);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          double v = a < 4 ? fma(kC, SS(a, i), kG * C[a][i])
+                                 : fma(kE, SS(el0[a < 4 ? 0 : a - 4], i) + SS(el1[a < 4 ? 0 : a - 4], i),
+                                       kG * E[a < 4 ? 0 : a - 4][i]);
+          const int rb = rw[3 * a + i];
+          v += lds_if(sin + (unsigned)(3 * pa + i) * 256u, ta);
+          sts_if(sout + (unsigned)(3 * a + i) * 256u, v, ha);
+          red_if(out + (rb + col), v, live && !ha && rb >= 0);
+        }
+      }
+    }
+    __syncwarp();
+    if (more) {
+      el++;
+      x++;
+    } else {
+      if (lane == 0 && next < ne) load(buf ^ 1, next);
+      el = __shfl_sync(FULL, next, 0);
+      x = 0;
     }
   }
 }
@@ -811,10 +771,10 @@ __global__ void k_tf_transient(const TfTrArgs T) {
 }
 
 // Residual of the condensed three-field element from its point records alone
-// (quadratic tets; the residual rows of k_assemble_p2m without its stiffness):
+// (quadratic tets; the residual part of k_assemble_p2r without its stiffness):
 // R_bi = sum_q sum_j (w tau_ij + w J s delta_ij) p_qb,j with p_qb = G_q^T dN_b/dxi,
 // s = c (sum w J - theta W) + kappa U'(theta) - P, c = kappa U''(theta) / W;
-// w tau = record fields 9..14 minus the geometric term h on the diagonal.
+// w tau = T' minus the geometric term h on the diagonal.
 // One thread per record slot (element perm[es]); inverted elements have zeroed
 // records (W = 0) and are skipped, as the assembly skips them.
 __global__ void k_tf_residual(const QpArgs A, const int *dof, double *R) {
@@ -825,11 +785,11 @@ __global__ void k_tf_residual(const QpArgs A, const int *dof, double *R) {
   const double *rec = A.qrec;
   double W = 0.0, SJ = 0.0;
   for (int q = 0; q < 4; q++) {
-    SJ += rec[yrec_idx<NRF>(es * 4 + q, 26)];
-    W += rec[yrec_idx<NRF>(es * 4 + q, 27)];
+    SJ += rec[(es * 4 + q) * NRF + kYWJ];
+    W += rec[(es * 4 + q) * NRF + kYW];
   }
   if (!(W > 0.0)) return;
-  const double th = rec[yrec_idx<NRF>(es * 4, 28)], Pe = rec[yrec_idx<NRF>(es * 4, 29)];
+  const double th = rec[es * 4 * NRF + kYTheta], Pe = rec[es * 4 * NRF + kYP];
   double dU, d2U;
   vol_derivs(A.mat.vol_pot, th, dU, d2U);
   const double c = A.mat.kappa * d2U / W;
@@ -839,10 +799,10 @@ __global__ void k_tf_residual(const QpArgs A, const int *dof, double *R) {
   for (int q = 0; q < 4; q++) {
     const long qs = es * 4 + q;
     double G[9], T[3][3];
-    for (int k = 0; k < 9; k++) G[k] = rec[yrec_idx<NRF>(qs, k)];
-    const double h = rec[yrec_idx<NRF>(qs, 25)], wJs = rec[yrec_idx<NRF>(qs, 26)] * sc;
+    for (int k = 0; k < 9; k++) G[k] = rec[qs * NRF + kYG + k];
+    const double h = rec[qs * NRF + kYH], wJs = rec[qs * NRF + kYWJ] * sc;
     double wt[6];
-    for (int k = 0; k < 6; k++) wt[k] = rec[yrec_idx<NRF>(qs, 9 + k)] - (k < 3 ? h : 0.0);
+    for (int k = 0; k < 6; k++) wt[k] = rec[qs * NRF + kYT + k] - (k < 3 ? h : 0.0);
     // Voigt order xx yy zz yz xz xy
     T[0][0] = wt[0] + wJs; T[1][1] = wt[1] + wJs; T[2][2] = wt[2] + wJs;
     T[1][2] = T[2][1] = wt[3];

@@ -21,7 +21,7 @@
 
 #include "assemble.cuh"
 #include "assemble_gather.cuh"
-#include "assemble_mma.cuh"
+#include "assemble_p2.cuh"
 #include "assemble_p1.cuh"
 #include "cm_integrate.cuh"
 #include "cp_crystal.cuh"
@@ -63,7 +63,7 @@ struct pgfem_gpu_ctx {
   long bytes = 0;
   double *qrec = nullptr;  // point records (kYRec x nqp for 10-node elements, kQRec x nqp for 4-node)
   int *eblk = nullptr;     // scatter blocks of 10-node elements (kEBW words each), processing order
-  // tensor-core quadratic-tet path: processing order (slot -> element), and a
+  // quadratic-tet path: processing order (slot -> element), and a
   // second stream with fork/join events on which K is zeroed while the point
   // kernel runs
   int *perm = nullptr;
@@ -94,7 +94,7 @@ struct pgfem_gpu_ctx {
   double *F0_tab = nullptr;
   int ngroups = 0;
   unsigned *sched_ticket = nullptr;
-  unsigned *p2m_ticket = nullptr;  // tile counter of the quadratic-tet assembly
+  unsigned *p2_ticket = nullptr;  // run counter of the quadratic-tet assembly
   // three-field (CM3F) element: pressure and volume per element (element
   // order), the expanded displacement increment of the local update, and the
   // record width the point records were allocated with
@@ -183,7 +183,7 @@ ShapeTable make_shape(int nne) {
     for (int a = 0; a < 4; a++) t.N[0][a] = 0.25;  // PGFem3D_N at the centroid
     return t;
   }
-  const double A = 0.58541020, B = 0.13819660;
+  const double A = kP2RuleA, B = kP2RuleB;
   const double k[4] = {A, B, B, B}, e[4] = {B, A, B, B}, z[4] = {B, B, A, B};
   for (int q = 0; q < 4; q++) {
     const double ksi = k[q], eta = e[q], zet = z[q];
@@ -345,7 +345,7 @@ void release(pgfem_gpu_ctx *c) {
                   c->colour_elems, c->qrec, c->eblk, c->perm,
                   c->cp_R, c->cp_F, c->cp_detJw, c->cp_out, c->cp_guess, c->cp_iters, c->cp_counter,
                   c->cp_Fn, c->cp_feat, c->cp_pred, c->cp_fallbacks, c->elem_group, c->F0_tab, c->cp_conv,
-                  c->sched_ticket, c->p2m_ticket, c->tf_P, c->tf_theta, c->tf_dunode, c->tf_inc, c->nbc_desc_tr, c->nbc_elem, c->nbc_feat, c->nbc_type, c->nbc_off, c->nbc_face,
+                  c->sched_ticket, c->p2_ticket, c->tf_P, c->tf_theta, c->tf_dunode, c->tf_inc, c->nbc_desc_tr, c->nbc_elem, c->nbc_feat, c->nbc_type, c->nbc_off, c->nbc_face,
                   c->nbc_load, c->tr_buf, c->state_nm1, c->tr_F, c->tf_hist, c->tf_mid, c->mass_csr, c->cp_rec, c->p1rec};
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -419,14 +419,13 @@ int launch_asm(const AsmArgs &a, long nitems, cudaStream_t s) {
 }
 
 // Point updates of all quadrature points into c->qrec (allocated on first use;
-// 26-double records for the tensor-core quadratic-tet kernel, 30 for its
+// 26-double records for the quadratic-tet assembly, 30 for its
 // three-field form, 38 for the linear-tet kernels).
 template <int NNE, int NQP, int MODEL, bool TF = false>
 int launch_qp_update(pgfem_gpu_ctx *c, cudaStream_t s, double wscale = 1.0) {
   constexpr bool YREC = NNE == 10;
   const int nf = YREC ? yrec_fields(TF) : kQRec;
-  // the tiled layout of the 10-node records is padded to whole tiles
-  const size_t npts = YREC ? (size_t)((c->nqp + kMPtsT - 1) / kMPtsT) * kMPtsT : (size_t)c->nqp;
+  const size_t npts = (size_t)c->nqp;
   if (c->qrec && c->qrec_fields < nf) {  // a wider record than allocated
     cudaFree(c->qrec);
     c->bytes -= (long)(sizeof(double) * c->qrec_fields * npts);
@@ -462,10 +461,7 @@ int launch_qp_update(pgfem_gpu_ctx *c, cudaStream_t s, double wscale = 1.0) {
   return PGFEM_GPU_OK;
 }
 
-// quadratic tets in two kernels: point updates into c->qrec (40-double
-// records; K zeroed meanwhile on the context's second stream), then the
-// tensor-core element assembly from the records
-// K's first write of the tensor-core quadratic-tet path, on the side stream: zeros, or
+// K's first write of the quadratic-tet path, on the side stream: zeros, or
 // k_c times `from` (nnz).
 int fork_K_init(pgfem_gpu_ctx *c, double *K, cudaStream_t s, const double *from = nullptr, double k_c = 0.0) {
   CK(cudaEventRecord(c->zfork, s));
@@ -476,15 +472,17 @@ int fork_K_init(pgfem_gpu_ctx *c, double *K, cudaStream_t s, const double *from 
   } else {
     CK(cudaMemsetAsync(K, 0, sizeof(double) * c->nnz, c->zstream));
   }
-  CK(cudaMemsetAsync(c->p2m_ticket, 0, sizeof(unsigned), c->zstream));
+  CK(cudaMemsetAsync(c->p2_ticket, 0, sizeof(unsigned), c->zstream));
   CK(cudaEventRecord(c->zjoin, c->zstream));
   return PGFEM_GPU_OK;
 }
 
+// Quadratic tets in two kernels: point updates into c->qrec (K zeroed meanwhile on the
+// context's second stream), then the element assembly from the records.
 // wscale: factor of the records' point weights; K_ready: the caller has called fork_K_init.
 template <int MODEL, bool TF = false>
-int launch_p2m(pgfem_gpu_ctx *c, const AsmArgs &a0, cudaStream_t s, double wscale = 1.0, bool K_ready = false) {
-  if (!TF && c->three_field) return launch_p2m<MODEL, true>(c, a0, s, wscale, K_ready);
+int launch_p2r(pgfem_gpu_ctx *c, const AsmArgs &a0, cudaStream_t s, double wscale = 1.0, bool K_ready = false) {
+  if (!TF && c->three_field) return launch_p2r<MODEL, true>(c, a0, s, wscale, K_ready);
   if (!K_ready)
     if (int r = fork_K_init(c, a0.K, s)) return r;
   if (int r = launch_qp_update<10, 4, MODEL, TF>(c, s, wscale)) return r;
@@ -492,21 +490,27 @@ int launch_p2m(pgfem_gpu_ctx *c, const AsmArgs &a0, cudaStream_t s, double wscal
   AsmArgs a = a0;
   a.qrec = c->qrec;
   a.eblk = c->eblk;
-  a.ticket = c->p2m_ticket;
-  const size_t smem = p2m_smem_bytes(TF);
-  auto kern = k_assemble_p2m<MODEL, TF>;
+  a.ticket = c->p2_ticket;
+  if (!g_num_sms) grid_for(1, 1, 1);
+  const size_t smem = p2r_smem_bytes(TF);
+  auto kern = k_assemble_p2r<MODEL, TF>;
   static bool attr_set = false;
   if (!attr_set) {
     CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_set = true;
   }
   int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kMThreads, smem));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kP2Threads, smem));
   if (per_sm < 1) per_sm = 1;
-  if (!g_num_sms) grid_for(1, 1, 1);
-  const long tiles = (a.ne + kMTE - 1) / kMTE;
-  const long grid = std::max<long>(1, std::min<long>(tiles, (long)g_num_sms * per_sm));
-  kern<<<(unsigned)grid, kMThreads, smem, s>>>(a);
+  // elements per run: the longest whose rounds over all warps cost at most 15 %
+  // more elements than the shortest's
+  const long warps = (long)g_num_sms * per_sm * (kP2Threads / 32);
+  auto rounds = [&](long r) { return (a.ne + r * warps - 1) / (r * warps) * r; };
+  int run = kP2Run;
+  while (run > 1 && (double)rounds(run) > 1.15 * (double)rounds(1)) run /= 2;
+  const long blocks = (a.ne + run * (kP2Threads / 32) - 1) / (run * (kP2Threads / 32));
+  const long grid = std::max<long>(1, std::min<long>(blocks, (long)g_num_sms * per_sm));
+  kern<<<(unsigned)grid, kP2Threads, smem, s>>>(a, run);
   CK(cudaGetLastError());
   return PGFEM_GPU_OK;
 }
@@ -620,9 +624,9 @@ int dispatch(pgfem_gpu_ctx *c, const AsmArgs &a, long nitems, cudaStream_t s) {
     return c->nne == 4 ? launch_asm<4, 1, 3, ATOMIC, WANT_K, DENSE>(a, nitems, s)
                        : launch_asm<10, 4, 3, ATOMIC, WANT_K, DENSE>(a, nitems, s);
   // quadratic tets, R+K into the CSR with atomic scatter over all elements:
-  // the point kernel + the tensor-core element assembly
+  // the point kernel + the element assembly
   if (c->nne == 10 && ATOMIC && WANT_K && !DENSE && !a.elist && a.R)
-    return c->model == PGFEM_MODEL_J2 ? launch_p2m<1>(c, a, s) : launch_p2m<0>(c, a, s);
+    return c->model == PGFEM_MODEL_J2 ? launch_p2r<1>(c, a, s) : launch_p2r<0>(c, a, s);
   // linear tets, R+K into the CSR with atomic scatter over all elements: the
   // point kernel + column-split assembly with the context's schedule
   if (c->nne == 4 && ATOMIC && WANT_K && !DENSE && !a.elist && a.R)
@@ -889,9 +893,9 @@ int launch_neumann(pgfem_gpu_ctx *c, double *d_R, double *d_K, cudaStream_t s, c
   return PGFEM_GPU_OK;
 }
 
-// Whether an R+K call of this context runs the tensor-core quadratic-tet
+// Whether an R+K call of this context runs the two-kernel quadratic-tet
 // path (the branch of dispatch() for 10-node elements, atomic scatter).
-bool uses_p2m(const pgfem_gpu_ctx *c) {
+bool uses_p2r(const pgfem_gpu_ctx *c) {
   return c->eblk && c->model != PGFEM_MODEL_CP && c->mat.dev_pot != 2 && c->scatter_mode == PGFEM_SCATTER_ATOMIC;
 }
 
@@ -907,8 +911,8 @@ bool gathers(const pgfem_gpu_ctx *c, const double *d_R, const double *d_K) {
 // One assembly on device buffers (zeroing R and K first).
 int assemble_device(pgfem_gpu_ctx *c, const double *d_u, const double *d_presc, double *d_R,
                     double *d_K, cudaStream_t s, double dt = 0.0) {
-  if (c->three_field) {  // the three-field element runs the tensor-core path only
-    if (!d_R || !uses_p2m(c)) return PGFEM_GPU_EINVAL;
+  if (c->three_field) {  // the three-field element runs the two-kernel path only
+    if (!d_R || !uses_p2r(c)) return PGFEM_GPU_EINVAL;
     if (!d_K) {  // residual only: the stiffness goes to a scratch K
       if (int r = ensure_K_scratch(c)) return r;
       d_K = c->d_K;
@@ -916,8 +920,8 @@ int assemble_device(pgfem_gpu_ctx *c, const double *d_u, const double *d_presc, 
   }
   const bool own = gathers(c, d_R, d_K);  // the row owners write every entry of R and K
   if (d_R && !own) CK(cudaMemsetAsync(d_R, 0, sizeof(double) * c->ndof, s));
-  // the tensor-core quadratic-tet path zeroes K itself, beside its point kernel
-  if (d_K && !own && !(uses_p2m(c) && d_R)) CK(cudaMemsetAsync(d_K, 0, sizeof(double) * c->nnz, s));
+  // the quadratic-tet path zeroes K itself, beside its point kernel
+  if (d_K && !own && !(uses_p2r(c) && d_R)) CK(cudaMemsetAsync(d_K, 0, sizeof(double) * c->nnz, s));
   if (!own || c->model == PGFEM_MODEL_CP || c->nbc_nface) {
     const long n3 = 3 * c->nn;
     k_expand_u<<<(unsigned)((n3 + 255) / 256), 256, 0, s>>>(c->dof, c->nn, d_u, d_presc, c->unode);
@@ -1161,7 +1165,7 @@ void build_colours(const pgfem_gpu_ctx *m, const std::vector<int> &conn, const s
   for (long e = 0; e < m->ne; e++) elems[fill[colour[e]]++] = (int)e;
 }
 
-// Element processing order of the tensor-core quadratic-tet kernel: columns
+// Element processing order of the quadratic-tet assembly: columns
 // of 6 x 6 element-size bins across the two shorter axes of the bounding
 // box, swept along the longest axis, bins in lexicographic order inside a
 // column (element centroids from the four vertex nodes; element size h =
@@ -1213,6 +1217,32 @@ std::vector<int> locality_order(const pgfem_mesh_desc *m) {
                    });
   std::vector<int> perm((size_t)ne);
   for (long e = 0; e < ne; e++) perm[e] = key[e].second;
+  // within a window of the order, the element that shares most corners with its
+  // predecessor goes next: consecutive elements hand each other shared entries
+  // (k_assemble_p2r), and element numberings need not chain faces
+  constexpr long kWin = 6;
+  struct Corners {
+    int n[4], e;
+  };
+  std::vector<Corners> q((size_t)ne);
+  for (long e = 0; e < ne; e++) {
+    for (int i = 0; i < 4; i++) q[e].n[i] = m->conn[(long)perm[e] * m->nne + i];
+    q[e].e = perm[e];
+  }
+  for (long e = 0; e + 1 < ne; e++) {
+    long best = e + 1;
+    int most = -1;
+    for (long x = e + 1; x < std::min(ne, e + 1 + kWin) && most < 3; x++) {
+      int n = 0;
+      for (int i = 0; i < 4; i++)
+        for (int j = 0; j < 4; j++) n += q[e].n[i] == q[x].n[j];
+      if (n > most) most = n, best = x;
+    }
+    const Corners b = q[best];
+    for (long x = best; x > e + 1; x--) q[x] = q[x - 1];
+    q[e + 1] = b;
+  }
+  for (long e = 0; e < ne; e++) perm[e] = q[e].e;
   return perm;
 }
 
@@ -1343,12 +1373,12 @@ int pgfem_gpu_create(const pgfem_mesh_desc *m, const pgfem_material_desc *mat, c
   }
   // linear tets: lists of the row owners
   if (m->nne == 4 && c->mat.dev_pot != 2 && (r = build_gather(c, dof, rowptr0, rowlen, mask))) return fail(r);
-  // tensor-core quadratic-tet path: processing order, scatter blocks in that
+  // quadratic-tet path: processing order, scatter blocks in that
   // order, the second stream that zeroes K
   if (m->nne == 10 && c->model != PGFEM_MODEL_CP && c->mat.dev_pot != 2) {
     std::vector<int> perm = locality_order(m);
     if ((r = upload(c, &c->perm, perm.data(), perm.size())) ||
-        (r = dalloc(c, &c->eblk, (size_t)((ne + kMTE - 1) / kMTE) * kMTE * kEBW)) || (r = dalloc(c, &c->p2m_ticket, 1)))
+        (r = dalloc(c, &c->eblk, (size_t)ne * kEBW)) || (r = dalloc(c, &c->p2_ticket, 1)))
       return fail(r);
     if (cudaStreamCreateWithFlags(&c->zstream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->zfork, cudaEventDisableTiming) != cudaSuccess ||
@@ -1429,7 +1459,7 @@ int pgfem_gpu_set_three_field(pgfem_gpu_ctx *c, const double *P, const double *t
     return PGFEM_GPU_OK;
   }
   if (!P || !theta) return PGFEM_GPU_EINVAL;
-  if (c->nne != 10 || (c->model != PGFEM_MODEL_HE && c->model != PGFEM_MODEL_J2) || !uses_p2m(c) ||
+  if (c->nne != 10 || (c->model != PGFEM_MODEL_HE && c->model != PGFEM_MODEL_J2) || !uses_p2r(c) ||
       c->elem_group)
     return PGFEM_GPU_EINVAL;
   for (long e = 0; e < c->ne; e++)
@@ -1640,7 +1670,7 @@ int pgfem_gpu_launches_per_assembly(const pgfem_gpu_ctx *c) {
   if (c->mat.dev_pot == 2)  // u expansion + per-node kernel launches (one per colour in colour mode)
     return 1 + (c->scatter_mode == PGFEM_SCATTER_COLOUR ? (int)c->colour_off.size() - 1 : 1) + nbc;
   if (c->nne == 10 && c->scatter_mode == PGFEM_SCATTER_ATOMIC)
-    return 3 + nbc;  // u expansion, point updates, tensor-core R+K assembly
+    return 3 + nbc;  // u expansion, point updates, R+K assembly
   if (c->nne == 4 && c->scatter_mode == PGFEM_SCATTER_ATOMIC)  // (u expansion,) point updates, R+K assembly
     return (c->gather && !c->nbc_nface ? 2 : 3) + nbc;
   const int nasm = c->scatter_mode == PGFEM_SCATTER_COLOUR ? (int)c->colour_off.size() - 1 : 1;
@@ -2310,7 +2340,7 @@ static int ensure_mass(pgfem_gpu_ctx *c, cudaStream_t s) {
 // condensation's and the inertia terms of R.  Against transient_3f and the passes of
 // transient_core it saves the pass over K (517 us), the older point's records and
 // residual (250 us) and the correction and inertia kernels (578 us) for one kernel of
-// 257 us that runs beside K's start: 3.01 -> 1.94 ms at 384,000 elements.  Surface
+// 257 us that runs beside K's start: 3.01 -> 1.94 ms at 384,000 elements, 1.66 ms with the assembly of k_assemble_p2r.  Surface
 // loads scale with their own times, so they keep transient_3f.
 static int transient_3f_fused(pgfem_gpu_ctx *c, const double *tu2, const double *tu1, const double *tu0,
                               const double *tp2, const double *tp1, const double *tp0, double alpha, double dt_np1,
@@ -2359,7 +2389,7 @@ static int transient_3f_fused(pgfem_gpu_ctx *c, const double *tu2, const double 
     CK(cudaEventCreate(&e1));
     CK(cudaEventRecord(e0, s));
   }
-  r = launch_p2m<PGFEM_MODEL_HE, true>(c, a, s, T.kK, true);
+  r = launch_p2r<PGFEM_MODEL_HE, true>(c, a, s, T.kK, true);
   if (e0) {
     CK(cudaEventRecord(e1, s));
     c->events.emplace_back(e0, e1);
@@ -2397,7 +2427,7 @@ static int transient_core(pgfem_gpu_ctx *c, const double *tu2, const double *tu1
     CK(cudaMemcpyAsync(c->nbc_desc_tr, d.data(), sizeof(double) * d.size(), cudaMemcpyHostToDevice, s));
     c->nbc_desc_cur = c->nbc_desc_tr;
   }
-  if (c->three_field && wantK && !c->nbc_nface && uses_p2m(c))
+  if (c->three_field && wantK && !c->nbc_nface && uses_p2r(c))
     return transient_3f_fused(c, tu2, tu1, tu0, tp2, tp1, tp0, alpha, dt_np1, dt_n, rho, s);
   if (c->three_field) {
     r = transient_3f(c, tu2, tu1, tu0, tp2, tp1, tp0, tua, tpa, tR2, alpha, dt_np1, dt_n, wantK, s);

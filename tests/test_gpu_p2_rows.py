@@ -1,0 +1,53 @@
+"""The quadratic-tet assembly (a warp per element, runs of elements that hand
+shared entries on) against the general assembly kernel (colour scatter) and
+the residual-only call: meshes below one run, of one run per warp and of
+several claims with a partial last run; elements in mesh order and shuffled
+(neighbours that share a face, an edge, a corner or nothing); J2 points elastic
+and yielding; local numberings rotated element by element.  The two differ in the order of the sums only; the tolerance is
+the one of the other parity tests."""
+import numpy as np
+import pytest
+
+import pgfem_gpu as pg
+import workloads as wl
+from test_gpu_parity import check_K, check_R
+
+pytestmark = pytest.mark.gpu
+
+
+def _rotate(conn, rng):
+    """Every element's nodes by a random even permutation of its corners."""
+    edge = {frozenset(v): i for i, v in enumerate([(0, 1), (1, 2), (0, 2), (0, 3), (1, 3), (2, 3)])}
+    even = [(0, 1, 2, 3), (1, 2, 0, 3), (2, 0, 1, 3), (1, 0, 3, 2), (2, 3, 0, 1), (3, 2, 1, 0), (0, 2, 3, 1), (0, 3, 1, 2)]
+    out = conn.copy()
+    for e, k in enumerate(rng.integers(0, len(even), len(conn))):
+        c = even[k]
+        out[e, :4] = conn[e, list(c)]
+        for (i, j), x in {(0, 1): 4, (1, 2): 5, (0, 2): 6, (0, 3): 7, (1, 3): 8, (2, 3): 9}.items():
+            out[e, x] = conn[e, 4 + edge[frozenset((c[i], c[j]))]]
+    return out
+
+
+@pytest.mark.parametrize("n,model,mixed", [(1, "j2", False), (2, "he", True), (5, "j2", True), (11, "he", False),
+                                           (15, "j2", True)])
+def test_matches_general_kernel(gpu, n, model, mixed):
+    p = wl.tension(n=n, nne=10, model=model, stretch=0.004, predictor=True)
+    rng = np.random.default_rng(n)
+    if mixed:
+        p.conn = np.ascontiguousarray(_rotate(p.conn[rng.permutation(len(p.conn))], rng))
+    p.X = p.X + 0.02 / n * rng.uniform(-1, 1, p.X.shape)
+    p.u = p.u + 2e-3 / n * rng.uniform(-1, 1, p.ndof)
+    ctx = p.context()
+    R, K, st = ctx.assemble_RK(p.u, p.u_presc)
+    assert st.ok(), st.as_dict()
+    g = p.context()
+    g.set_scatter_mode(pg.SCATTER_COLOUR)
+    Rg, Kg, st = g.assemble_RK(p.u, p.u_presc)
+    assert st.ok()
+    check_R(R, Rg)
+    check_K(K, Kg, p.Ap)
+    R2, K2, _ = ctx.assemble_RK(p.u, p.u_presc)  # a second call on the same context
+    check_R(R2, Rg)
+    check_K(K2, Kg, p.Ap)
+    ctx.close()
+    g.close()
