@@ -88,6 +88,7 @@ struct AsmArgs {
   // test switch: the producer withholds its first hand-off
   unsigned long long wait_ns;
   int stall;
+  bool K_zeroed;  // quadratic tets, host: K was zeroed on the assembly's stream
   double rscale;  // quadratic tets: factor of the residual against the records' (1: the quasi-static calls)
   Mat mat;
   ShapeTable shp;

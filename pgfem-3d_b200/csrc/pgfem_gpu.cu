@@ -279,6 +279,24 @@ __global__ void k_expand_u(const int *dof, long nn, const double *u, const doubl
   unode[n] = id > 0 ? u[id - 1] : (id < 0 && presc ? presc[-id - 1] : 0.0);
 }
 
+// k_expand_u with the zero fills of R (ndof), of K (nnz; nullptr: not this one) and of the
+// run counter: one launch in place of up to four and the second stream's fork and join.
+__global__ void __launch_bounds__(256) k_expand_u_zero(const int *__restrict__ dof, long nn,
+                                                       const double *__restrict__ u,
+                                                       const double *__restrict__ presc, double *__restrict__ unode,
+                                                       double *__restrict__ R, long ndof, double *__restrict__ K,
+                                                       long nnz, unsigned *ticket) {
+  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x, nt = (long)gridDim.x * blockDim.x;
+  if (t == 0) *ticket = 0;
+  for (long n = t; n < 3 * nn; n += nt) {
+    const int id = dof[n];
+    unode[n] = id > 0 ? u[id - 1] : (id < 0 && presc ? presc[-id - 1] : 0.0);
+  }
+  for (long n = t; n < ndof; n += nt) R[n] = 0.0;
+  if (K)
+    for (long n = t; n < nnz; n += nt) K[n] = 0.0;
+}
+
 // Element->CSR node-block map: for each element and node pair (a, b), the
 // column position of node b's first free DOF inside the rows of node a,
 // checked against the caller's pattern (all free columns of b present and
@@ -463,7 +481,8 @@ int launch_qp_update(pgfem_gpu_ctx *c, cudaStream_t s, double wscale = 1.0) {
 
 // K's first write of the quadratic-tet path, on the side stream: zeros, or
 // k_c times `from` (nnz).
-int fork_K_init(pgfem_gpu_ctx *c, double *K, cudaStream_t s, const double *from = nullptr, double k_c = 0.0) {
+int fork_K_init(pgfem_gpu_ctx *c, double *K, cudaStream_t s, bool zero_ticket, const double *from = nullptr,
+                double k_c = 0.0) {
   CK(cudaEventRecord(c->zfork, s));
   CK(cudaStreamWaitEvent(c->zstream, c->zfork, 0));
   if (from) {
@@ -472,21 +491,20 @@ int fork_K_init(pgfem_gpu_ctx *c, double *K, cudaStream_t s, const double *from 
   } else {
     CK(cudaMemsetAsync(K, 0, sizeof(double) * c->nnz, c->zstream));
   }
-  CK(cudaMemsetAsync(c->p2_ticket, 0, sizeof(unsigned), c->zstream));
+  if (zero_ticket) CK(cudaMemsetAsync(c->p2_ticket, 0, sizeof(unsigned), c->zstream));
   CK(cudaEventRecord(c->zjoin, c->zstream));
   return PGFEM_GPU_OK;
 }
 
 // Quadratic tets in two kernels: point updates into c->qrec (K zeroed meanwhile on the
 // context's second stream), then the element assembly from the records.
-// wscale: factor of the records' point weights; K_ready: the caller has called fork_K_init.
+// wscale: factor of the records' point weights.  K and the run counter: zeroed by the caller
+// on s (small K) or written by its fork_K_init, whose stream is joined here.
 template <int MODEL, bool TF = false>
-int launch_p2r(pgfem_gpu_ctx *c, const AsmArgs &a0, cudaStream_t s, double wscale = 1.0, bool K_ready = false) {
-  if (!TF && c->three_field) return launch_p2r<MODEL, true>(c, a0, s, wscale, K_ready);
-  if (!K_ready)
-    if (int r = fork_K_init(c, a0.K, s)) return r;
+int launch_p2r(pgfem_gpu_ctx *c, const AsmArgs &a0, cudaStream_t s, double wscale = 1.0) {
+  if (!TF && c->three_field) return launch_p2r<MODEL, true>(c, a0, s, wscale);
   if (int r = launch_qp_update<10, 4, MODEL, TF>(c, s, wscale)) return r;
-  CK(cudaStreamWaitEvent(s, c->zjoin, 0));
+  if (!a0.K_zeroed) CK(cudaStreamWaitEvent(s, c->zjoin, 0));
   AsmArgs a = a0;
   a.qrec = c->qrec;
   a.eblk = c->eblk;
@@ -919,10 +937,25 @@ int assemble_device(pgfem_gpu_ctx *c, const double *d_u, const double *d_presc, 
     }
   }
   const bool own = gathers(c, d_R, d_K);  // the row owners write every entry of R and K
-  if (d_R && !own) CK(cudaMemsetAsync(d_R, 0, sizeof(double) * c->ndof, s));
-  // the quadratic-tet path zeroes K itself, beside its point kernel
-  if (d_K && !own && !(uses_p2r(c) && d_R)) CK(cudaMemsetAsync(d_K, 0, sizeof(double) * c->nnz, s));
-  if (!own || c->model == PGFEM_MODEL_CP || c->nbc_nface) {
+  const bool p2 = d_K && d_R && uses_p2r(c);
+  // the quadratic-tet path zeroes a small K with the displacements (a fork and join of
+  // the second stream costs more than 16 MB of stores: 2,058 elements, 6.6 MB, 26.7 ->
+  // 24.1 us per call; 384 elements, 29 -> 19 us), a larger one on the second stream
+  // beside its point kernel
+  const bool K_zeroed = p2 && (size_t)c->nnz * sizeof(double) <= (16u << 20);
+  if (d_R && !own && !p2) CK(cudaMemsetAsync(d_R, 0, sizeof(double) * c->ndof, s));
+  if (d_K && !own && !p2) CK(cudaMemsetAsync(d_K, 0, sizeof(double) * c->nnz, s));
+  if (p2) {
+    const long n3 = 3 * c->nn;
+    const long work = std::max<long>(n3, K_zeroed ? c->nnz / 4 : 0);
+    if (!g_num_sms) grid_for(1, 1, 1);
+    const long grid = std::max<long>((n3 + 255) / 256, std::min<long>((work + 255) / 256, (long)g_num_sms * 8));
+    k_expand_u_zero<<<(unsigned)grid, 256, 0, s>>>(c->dof, c->nn, d_u, d_presc, c->unode, d_R, c->ndof,
+                                                   K_zeroed ? d_K : nullptr, c->nnz, c->p2_ticket);
+    CK(cudaGetLastError());
+    if (!K_zeroed)
+      if (int r = fork_K_init(c, d_K, s, false)) return r;
+  } else if (!own || c->model == PGFEM_MODEL_CP || c->nbc_nface) {
     const long n3 = 3 * c->nn;
     k_expand_u<<<(unsigned)((n3 + 255) / 256), 256, 0, s>>>(c->dof, c->nn, d_u, d_presc, c->unode);
     CK(cudaGetLastError());
@@ -942,6 +975,7 @@ int assemble_device(pgfem_gpu_ctx *c, const double *d_u, const double *d_presc, 
   AsmArgs a = base_args(c);
   a.R = d_R;
   a.K = d_K;
+  a.K_zeroed = K_zeroed;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (c->timing && c->events.size() < 4096) {
     CK(cudaEventCreate(&e0));
@@ -2352,7 +2386,7 @@ static int transient_3f_fused(pgfem_gpu_ctx *c, const double *tu2, const double 
   const long n3 = 3 * c->nn;
   double *ub = c->tf_mid + (size_t)4 * c->ne, *v = ub + n3;
   CK(cudaMemsetAsync(c->d_R, 0, sizeof(double) * c->ndof, s));
-  if ((r = fork_K_init(c, c->d_K, s, c->mass_csr, rho / dt_np1))) return r;
+  if ((r = fork_K_init(c, c->d_K, s, true, c->mass_csr, rho / dt_np1))) return r;
   k_tf_mid<<<ge, 128, 0, s>>>(c->ne, c->tf_P, c->tf_theta, c->tf_hist, alpha, c->tf_mid);
   k_tr_nodes<<<(unsigned)((n3 + 255) / 256), 256, 0, s>>>(c->dof, n3, tu2, tu1, tu0, c->npres ? tp2 : nullptr, tp1, tp0,
                                                           alpha, dt_np1, dt_n, c->unode, ub, v);
@@ -2389,7 +2423,7 @@ static int transient_3f_fused(pgfem_gpu_ctx *c, const double *tu2, const double 
     CK(cudaEventCreate(&e1));
     CK(cudaEventRecord(e0, s));
   }
-  r = launch_p2r<PGFEM_MODEL_HE, true>(c, a, s, T.kK, true);
+  r = launch_p2r<PGFEM_MODEL_HE, true>(c, a, s, T.kK);
   if (e0) {
     CK(cudaEventRecord(e1, s));
     c->events.emplace_back(e0, e1);
