@@ -105,6 +105,12 @@ struct Tile<10> {
   static constexpr int TE = 12;
 };
 
+// Programmatic dependent launch (linear tets; small quadratic-tet systems): a kernel lets the next
+// one of its call start while it runs, and waits for the previous one's results
+// before it touches memory.  Both are no-ops in a plain launch.
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ int rank_of(unsigned mask, int c) {
   return __popc(mask & ((1u << c) - 1u));
 }

@@ -198,6 +198,7 @@ struct P1PointArgs {
 template <int MODEL>
 __global__ void __launch_bounds__(128, 5) k_p1_points(const P1PointArgs A) {
   constexpr bool PLASTIC = MODEL == 1;
+  pdl_release();
   __shared__ double srow[128 * (kP1Rec + 1)];
   const long e0 = blockIdx.x * 128L, e = e0 + threadIdx.x;
   double *r = srow + threadIdx.x * (kP1Rec + 1);
@@ -437,6 +438,7 @@ __global__ void __launch_bounds__(128, MODEL == 2 ? 3 : 4) k_gather_p1(const Gat
   const int zero = gather_zero(A.L.most);
   const int crec = lane / NC, cch = lane - crec * NC;  // record and 16-byte word this lane copies
   const unsigned sdst = (unsigned)__cvta_generic_to_shared(stg + crec * ST + 2 * cch);
+  pdl_wait();
   const long step = (long)gridDim.x * nw;
   long gn = A.ticket ? 0 : (long)blockIdx.x * nw + warp, ge = 0;
   auto next = [&]() -> long {

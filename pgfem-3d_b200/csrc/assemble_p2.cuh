@@ -221,6 +221,10 @@ __device__ __forceinline__ void qp_point(const QpArgs &A, long qs, double *rec) 
 
 template <int NNE, int NQP, int MODEL, bool YREC = false, bool TF = false>
 __global__ void __launch_bounds__(128) k_qp_update(const QpArgs A) {
+  if (YREC) {
+    pdl_wait();
+    pdl_release();
+  }
   const long qs = blockIdx.x * (long)blockDim.x + threadIdx.x;  // record slot
   if (!YREC) {
     if (qs < A.nqp) qp_point<NNE, NQP, MODEL, YREC, TF>(A, qs, A.qrec);
@@ -402,6 +406,7 @@ __global__ void __launch_bounds__(kP2Threads, 3) k_assemble_p2r(const AsmArgs ar
   // neighbouring elements of the processing order and the CSR rows they reduce
   // into stay in L2 between neighbouring elements' contributions.
   const bool claims = (long)gridDim.x * NW * run < ne;
+  pdl_wait();
   long el = ((long)blockIdx.x * NW + warp) * run, next = ne;  // next: lane 0's claim
   if (claims) {
     if (lane == 0) el = (long)atomicAdd(args.ticket, 1u) * run;

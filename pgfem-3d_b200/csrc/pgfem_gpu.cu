@@ -286,6 +286,7 @@ __global__ void __launch_bounds__(256) k_expand_u_zero(const int *__restrict__ d
                                                        const double *__restrict__ presc, double *__restrict__ unode,
                                                        double *__restrict__ R, long ndof, double *__restrict__ K,
                                                        long nnz, unsigned *ticket) {
+  pdl_release();
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x, nt = (long)gridDim.x * blockDim.x;
   if (t == 0) *ticket = 0;
   for (long n = t; n < 3 * nn; n += nt) {
@@ -436,11 +437,29 @@ int launch_asm(const AsmArgs &a, long nitems, cudaStream_t s) {
   return PGFEM_GPU_OK;
 }
 
+// Kernel launch; pdl: it may start while the previous kernel of the stream runs (both use
+// griddepcontrol).
+template <class... P, class... A>
+cudaError_t launch_after(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, bool pdl,
+                         A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 // Point updates of all quadrature points into c->qrec (allocated on first use;
 // 26-double records for the quadratic-tet assembly, 30 for its
 // three-field form, 38 for the linear-tet kernels).
 template <int NNE, int NQP, int MODEL, bool TF = false>
-int launch_qp_update(pgfem_gpu_ctx *c, cudaStream_t s, double wscale = 1.0) {
+int launch_qp_update(pgfem_gpu_ctx *c, cudaStream_t s, double wscale = 1.0, bool pdl = false) {
   constexpr bool YREC = NNE == 10;
   const int nf = YREC ? yrec_fields(TF) : kQRec;
   const size_t npts = (size_t)c->nqp;
@@ -474,8 +493,7 @@ int launch_qp_update(pgfem_gpu_ctx *c, cudaStream_t s, double wscale = 1.0) {
   q.tf_P = c->tf_P;
   q.tf_theta = c->tf_theta;
   q.wscale = wscale;
-  k_qp_update<NNE, NQP, MODEL, YREC, TF><<<(unsigned)((c->nqp + 127) / 128), 128, 0, s>>>(q);
-  CK(cudaGetLastError());
+  CK(launch_after(k_qp_update<NNE, NQP, MODEL, YREC, TF>, (unsigned)((c->nqp + 127) / 128), 128, 0, s, pdl, q));
   return PGFEM_GPU_OK;
 }
 
@@ -503,7 +521,7 @@ int fork_K_init(pgfem_gpu_ctx *c, double *K, cudaStream_t s, bool zero_ticket, c
 template <int MODEL, bool TF = false>
 int launch_p2r(pgfem_gpu_ctx *c, const AsmArgs &a0, cudaStream_t s, double wscale = 1.0) {
   if (!TF && c->three_field) return launch_p2r<MODEL, true>(c, a0, s, wscale);
-  if (int r = launch_qp_update<10, 4, MODEL, TF>(c, s, wscale)) return r;
+  if (int r = launch_qp_update<10, 4, MODEL, TF>(c, s, wscale, a0.K_zeroed)) return r;
   if (!a0.K_zeroed) CK(cudaStreamWaitEvent(s, c->zjoin, 0));
   AsmArgs a = a0;
   a.qrec = c->qrec;
@@ -528,8 +546,7 @@ int launch_p2r(pgfem_gpu_ctx *c, const AsmArgs &a0, cudaStream_t s, double wscal
   while (run > 1 && (double)rounds(run) > 1.15 * (double)rounds(1)) run /= 2;
   const long blocks = (a.ne + run * (kP2Threads / 32) - 1) / (run * (kP2Threads / 32));
   const long grid = std::max<long>(1, std::min<long>(blocks, (long)g_num_sms * per_sm));
-  kern<<<(unsigned)grid, kP2Threads, smem, s>>>(a, run);
-  CK(cudaGetLastError());
+  CK(launch_after(kern, (unsigned)grid, kP2Threads, smem, s, a.K_zeroed, a, run));
   return PGFEM_GPU_OK;
 }
 
@@ -603,8 +620,10 @@ int launch_gather(pgfem_gpu_ctx *c, const double *rec, double *R, double *K, cud
   }
   const long need = (c->gl.ng + nw - 1) / nw;
   const long grid = std::max<long>(1, std::min<long>(need, (long)g_num_sms * c->g_per_sm[sel]));
-  kern<<<(unsigned)grid, 32 * nw, smem, s>>>(a);
-  CK(cudaGetLastError());
+  // behind k_p1_points the start overlaps on small meshes (6,000 elements: 14.3 -> 12.3 us a
+  // call); a launch is under 1 % of a call above
+  const bool pdl = MODEL != 2 && !a.ticket && c->ne <= (1L << 17);
+  CK(launch_after(kern, (unsigned)grid, 32 * nw, smem, s, pdl, a));
   return PGFEM_GPU_OK;
 }
 
@@ -940,8 +959,9 @@ int assemble_device(pgfem_gpu_ctx *c, const double *d_u, const double *d_presc, 
   const bool p2 = d_K && d_R && uses_p2r(c);
   // the quadratic-tet path zeroes a small K with the displacements (a fork and join of
   // the second stream costs more than 16 MB of stores: 2,058 elements, 6.6 MB, 26.7 ->
-  // 24.1 us per call; 384 elements, 29 -> 19 us), a larger one on the second stream
-  // beside its point kernel
+  // 24.1 us per call; 384 elements, 29 -> 19 us; and then the three kernels start
+  // before their predecessors end: 21.3 and 17.8 us), a larger one on the second
+  // stream beside its point kernel
   const bool K_zeroed = p2 && (size_t)c->nnz * sizeof(double) <= (16u << 20);
   if (d_R && !own && !p2) CK(cudaMemsetAsync(d_R, 0, sizeof(double) * c->ndof, s));
   if (d_K && !own && !p2) CK(cudaMemsetAsync(d_K, 0, sizeof(double) * c->nnz, s));

@@ -51,3 +51,32 @@ def test_matches_general_kernel(gpu, n, model, mixed):
     check_K(K2, Kg, p.Ap)
     ctx.close()
     g.close()
+
+
+@pytest.mark.parametrize("n,three_field", [(2, False), (3, True), (11, False)])
+def test_graph_replays_the_call(gpu, n, three_field):
+    """The captured call (programmatic launches below 16 MB of K, the second
+    stream's fork and join above) equals the direct one; replayed twice."""
+    import torch
+
+    p = wl.tension(n=n, nne=10, model="he", stretch=0.004, predictor=True)
+    ctx = p.context()
+    if three_field:
+        ne = len(p.conn)
+        ctx.set_three_field(np.full(ne, 3.0), np.full(ne, 1.001))
+    R, K, st = ctx.assemble_RK(p.u, p.u_presc)
+    assert st.ok()
+    d_u = torch.from_numpy(p.u).cuda()
+    d_p = torch.from_numpy(p.u_presc).cuda()
+    d_R = torch.full((p.ndof,), 7.0, dtype=torch.float64, device="cuda")
+    d_K = torch.full((p.nnz,), 7.0, dtype=torch.float64, device="cuda")
+    g = ctx.graph_create(d_u.data_ptr(), d_p.data_ptr(), d_R.data_ptr(), d_K.data_ptr())
+    s = torch.cuda.current_stream()
+    for _ in range(2):
+        d_K.fill_(5.0)
+        g.launch(s.cuda_stream)
+    torch.cuda.synchronize()
+    check_R(d_R.cpu().numpy(), R)
+    check_K(d_K.cpu().numpy(), K, p.Ap)
+    g.destroy()
+    ctx.close()
