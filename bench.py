@@ -177,7 +177,7 @@ def measured_hbm_gbs():
 def traffic_per_launch():
     """dram bytes of one R+K iterate's two kernels (point updates, then the
     assembly) from the committed ncu summary of the J2 quadratic-tet workload."""
-    path = os.path.join(ROOT, "profiles", "k_assemble_p2m_j2_p2_traffic.txt")
+    path = os.path.join(ROOT, "profiles", "k_assemble_p2r_j2_p2_traffic.txt")
     if not os.path.exists(path):
         return None
     for ln in open(path):
@@ -316,7 +316,7 @@ def run_ours(args, ws, rank, local):
         roof = {"bound": "hbm", "achieved": nbytes / (k_ms * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                 "peak_source": hbm_src}
     roof["frac"] = roof["achieved"] / roof["peak"]
-    roof["kernel"] = ("k_assemble<4,1,0> (fused R+K)" if he else
+    roof["kernel"] = ("k_p1_points<0> + k_gather_p1 (point updates, then the rows of R and K by their owners)" if he else
                       "k_qp_update<10,4,0,1,1> + k_assemble_p2r<0,1> (three-field point updates, then the condensed "
                       "R+K, a warp per element)" if tf else
                       "k_qp_update<10,4,1,1> + k_assemble_p2r<1> (point updates, then R+K, a warp per element)")
@@ -380,7 +380,7 @@ def cp_roofline(kernel_ms, iters, nqp, fp64_peak):
     ach = flops / (kernel_ms * 1e-3) / 1e12
     return {"bound": "fp64", "achieved": ach, "peak": fp64_peak, "unit": "TFLOP/s",
             "peak_source": "measured this run (FP64 FMA-chain probe, every SM)", "frac": ach / fp64_peak,
-            "traffic": None, "kernel": "k_cp_update (local Newton)", "kernel_ms": kernel_ms, "alg_flops": flops,
+            "traffic": None, "kernel": "k_cp_update_cx (local Newton and tangent, crystal frame)", "kernel_ms": kernel_ms, "alg_flops": flops,
             "flop_model": "%.0f per Newton iteration + %.0f per point" % (FLOP_CP_ITER, FLOP_CP_POINT)}
 
 
@@ -867,13 +867,10 @@ def run_nr(args, ws, rank, local):
             "alg_bytes": spmv_bytes, "traffic": None}
     roof["frac"] = roof["achieved"] / roof["peak"]
     # kernels of one step: per assembly its kernels + the norm (2); per solve the
-    # negation, the diagonal scaling and the final residual (5); per GMRES cycle
-    # 6; per queued Arnoldi step 11 (steps are queued 8 at a time, so a cycle
-    # queues at most 7 beyond its last step)
+    # negation, the diagonal scaling, the final residual (3), the update of u and at
+    # least one launch of the GMRES cycles
     solves = info.iters
-    cycles = solves + info.lin_iters // max(args.nr_kdim, 1)
-    launches = (info.iters + 1) * (ctx.launches_per_assembly() + 2) + 5 * solves + 6 * cycles \
-        + 11 * (info.lin_iters + 7 * cycles)
+    launches = (info.iters + 1) * (ctx.launches_per_assembly() + 2) + 7 * solves
     out = {"metric": NR_METRIC, "value": 1e3 / ms_step, "unit": "steps/s", "n_gpus": ws, "steps": nsteps,
            "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
            "vs_baseline": None, "dtype": "f64", "data": "synthetic (structured mesh, uniaxial tension)",
