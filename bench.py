@@ -367,12 +367,13 @@ def run_ours(args, ws, rank, local):
     return out
 
 
-# Declared FP64 work of the CP local update (survey figures for this model):
-# one Newton iteration (residual with 12 power laws at 40 flop each, 10x10
-# Jacobian, LU solve, one line-search residual) and the per-point fixed work
-# (set-up, consistent dM/dF with 9 right-hand sides).
-FLOP_CP_ITER = 10.0e3
-FLOP_CP_POINT = 8.0e3
+# Declared FP64 work of the CP local update in the crystal frame: one Newton
+# iteration (residual with 12 power laws, the reduced 6x6 Jacobian, its solve, one
+# line-search residual) and the per-point fixed work (set-up, consistent tangent
+# from the reduced Jacobian).  The sample-frame form with ten unknowns took 10e3
+# and 8e3.
+FLOP_CP_ITER = 1.3e3
+FLOP_CP_POINT = 7.0e3
 
 
 def cp_roofline(kernel_ms, iters, nqp, fp64_peak):
@@ -380,7 +381,8 @@ def cp_roofline(kernel_ms, iters, nqp, fp64_peak):
     ach = flops / (kernel_ms * 1e-3) / 1e12
     return {"bound": "fp64", "achieved": ach, "peak": fp64_peak, "unit": "TFLOP/s",
             "peak_source": "measured this run (FP64 FMA-chain probe, every SM)", "frac": ach / fp64_peak,
-            "traffic": None, "kernel": "k_cp_update_cx (local Newton and tangent, crystal frame)", "kernel_ms": kernel_ms, "alg_flops": flops,
+            "traffic": None, "kernel": "k_cp_update_cx (local Newton and tangent, crystal frame)", "kernel_ms": kernel_ms,
+            "alg_flops": flops,
             "flop_model": "%.0f per Newton iteration + %.0f per point" % (FLOP_CP_ITER, FLOP_CP_POINT)}
 
 
@@ -1016,7 +1018,7 @@ def run_transient(args, ws, rank, local):
            "config": {"workload": ("crystal plasticity, linear tets, %d^3 cells x 6 (%d elements), transient R+K "
                                    "with the mid-point plastic state" % (args.cp_n, p.ne)) if cp else
                                   ("three-field neo-Hookean, quadratic tets, %d^3 cells x 6 (%d elements, %d qp, "
-                                   "%d nnz), transient R+K: two condensed assemblies + correction + inertia"
+                                   "%d nnz), transient R+K: condensed assembly, older-point, condensation and inertia terms"
                                    % (args.n, p.ne, nqp, p.nnz)),
                       "alpha": alpha, "dt": [dt1, dt0], "rho": rho, "quasi_static_ms": ms_qs,
                       "transient_over_quasi_static": ms / ms_qs,
