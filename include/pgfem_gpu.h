@@ -180,7 +180,10 @@ int pgfem_gpu_set_neumann_load_history(pgfem_gpu_ctx *ctx, int nfeature, const d
  * three_field_update_device: the same on device buffers; with d_out NULL the
  * increments are added to the context's P and theta (what the device Newton
  * step, pgfem_gpu_newton_step, does after each solve while three-field is on),
- * else written to d_out (2 ne: dP, then d_theta). */
+ * else written to d_out (2 ne: dP, then d_theta).  Enqueued on stream (NULL: the
+ * default stream, as pgfem_gpu_assemble_RK_device); work of the context that
+ * another stream enqueues afterwards is the caller's to order, except that after
+ * a call on the default stream get_three_field and the host-buffer calls wait. */
 int pgfem_gpu_set_three_field(pgfem_gpu_ctx *ctx, const double *P, const double *theta);
 int pgfem_gpu_get_three_field(pgfem_gpu_ctx *ctx, double *P, double *theta);
 int pgfem_gpu_three_field_enabled(const pgfem_gpu_ctx *ctx);

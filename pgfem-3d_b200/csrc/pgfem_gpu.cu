@@ -1565,7 +1565,10 @@ __global__ void k_tf_apply(long ne, const double *inc, double *P, double *theta)
 int pgfem_gpu_three_field_update_device(pgfem_gpu_ctx *c, const double *d_u, const double *d_presc,
                                         const double *d_du, double *d_out, void *stream) {
   if (!c || !c->three_field || (c->ndof && (!d_u || !d_du)) || (c->npres && !d_presc)) return PGFEM_GPU_EINVAL;
-  cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
+  // the caller's stream, NULL the default one: d_u and d_du come from it and the next
+  // assembly on it reads P and theta (and writes c->unode); the context's own stream
+  // does not wait for the default stream
+  cudaStream_t s = (cudaStream_t)stream;
   int r;
   if (!c->tf_dunode && ((r = dalloc(c, &c->tf_dunode, 3 * c->nn)) || (r = dalloc(c, &c->tf_inc, 2 * c->ne))))
     return r;
@@ -1589,6 +1592,10 @@ int pgfem_gpu_three_field_update_device(pgfem_gpu_ctx *c, const double *d_u, con
   k_tf_update<<<g, 128, 0, s>>>(q, c->tf_dunode, inc, inc + c->ne);
   if (!d_out) k_tf_apply<<<g, 128, 0, s>>>(c->ne, inc, c->tf_P, c->tf_theta);
   CK(cudaGetLastError());
+  if (!s) {  // get_three_field and the host-buffer calls after it read P and theta on the context's stream
+    CK(cudaEventRecord(c->zfork, s));
+    CK(cudaStreamWaitEvent(c->stream, c->zfork, 0));
+  }
   return PGFEM_GPU_OK;
 }
 
