@@ -485,7 +485,7 @@ typedef struct {
   int maxit;       /* iteration cap (the reference's -maxit, default 1000) */
   int kdim;        /* GMRES restart length (-kdim, default 500); the basis takes (kdim + 1) * nrows doubles */
   double tol;      /* relative residual ||b - K x|| / ||b|| to reach (sol->err) */
-  int check_every; /* BiCGSTAB: iterations queued between host convergence checks; <= 0: 8 */
+  int check_every; /* BiCGSTAB, GMRES of large systems: iterations queued between host convergence checks; <= 0: 8 */
 } pgfem_solver_opts;
 
 typedef struct {
@@ -508,8 +508,9 @@ long pgfem_gpu_solver_device_bytes(const pgfem_gpu_solver *solver);
 /* y = K x on `stream` (device pointers; asynchronous). */
 int pgfem_gpu_spmv(pgfem_gpu_solver *solver, const double *d_K, const double *d_x, double *d_y, void *stream);
 /* K x = b by the solver's method; d_x holds the initial guess on entry.
- * Synchronises `stream` at each convergence check (GMRES: once per launch of
- * restart cycles; ETIMEOUT when a grid-wide wait of that kernel ran out). */
+ * Synchronises `stream` at each convergence check (GMRES up to about 3 M rows:
+ * once per launch of restart cycles; ETIMEOUT when a grid-wide wait of that kernel
+ * ran out). */
 int pgfem_gpu_solve(pgfem_gpu_solver *solver, const double *d_K, const double *d_b, double *d_x,
                     pgfem_solve_info *info, void *stream);
 

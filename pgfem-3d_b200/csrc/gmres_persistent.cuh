@@ -18,11 +18,11 @@
 // terms cancel.  The Givens rotations of a column run in one warp of CTA 0
 // beside the next product.
 //
-// Measured, us per step, against the launch sequence this replaces (ten launches
-// a step, rotations and back substitution in one-thread kernels), J2 quadratic
-// tets, kdim 100: 1,863 rows 70.5 -> 12.7, 13,583 rows 75.5 -> 14.2, 44,375 rows
-// 86 -> 27, 103,455 rows 122 -> 71, 343,343 rows 294 -> 238; kdim 500, 13,583 rows
-// 165 -> 28.  Up to some 30 k rows at kdim 100 (basis slice in shared memory) it
+// Measured, us per step, against the launch sequence that takes the large systems
+// (ten launches a step, rotations and back substitution in one-thread kernels;
+// solver.cu has the line between the two), J2 quadratic tets, kdim 100: 1,863 rows
+// 70.5 -> 12.7, 13,583 rows 75.5 -> 14.2, 44,375 rows 86 -> 27, 103,455 rows 122 -> 71,
+// 343,343 rows 294 -> 238; kdim 500, 13,583 rows 165 -> 28.  Up to some 30 k rows at kdim 100 (basis slice in shared memory) it
 // is bound by the five one-way messages of a step, about 1.3 us each between
 // SMs; above, by reading the basis four times a step from L2 and HBM.
 #pragma once
@@ -56,7 +56,7 @@ struct Args {
   unsigned long long wait_ns;
 };
 
-inline size_t smem_fixed(int rows, int m) {  // w, two columns of sums, rotations, the own Hessenberg column
+constexpr size_t smem_fixed(int rows, int m) {  // w, two columns of sums, rotations, the own Hessenberg column
   return sizeof(double) * ((size_t)rows + 2 * (m + 2) + 3 * (size_t)(m + 2) + kWarps + 1 + kThreads);
 }
 
