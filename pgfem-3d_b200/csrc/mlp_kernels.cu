@@ -74,7 +74,9 @@ int check_dev() {
 int set_smem_attrs() {
   static bool done = false;
   if (done) return PGFEM_GPU_OK;
-  MCK(cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInfSmem));
+  MCK(cudaFuncSetAttribute(k_mlp_forward<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)InfLayout<1>::smem));
+  MCK(cudaFuncSetAttribute(k_mlp_forward<kSlots>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)InfLayout<kSlots>::smem));
   MCK(cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem));
   done = true;
   return PGFEM_GPU_OK;
@@ -300,7 +302,14 @@ int pgfem_mlp_predict_device(pgfem_mlp *m, long n, const float *d_x, float *d_y,
   pgb::mlp::MlpDev dv = m->dev_view();
   dv.stall = m->stall;
   m->stall = 0;
-  k_mlp_forward<<<grid, kInfThreads, kInfSmem, (cudaStream_t)stream>>>(dv, n, d_x, d_y);
+  // one tile a CTA: one slot, which sets up a third of the threads, feature buffers and
+  // TMEM columns (us, one slot / three: 32 rows 18.5 / 20.5, 3,000 rows 18.5 / 22.2,
+  // 18,944 rows 18.5 / 22.5); from the second tile a CTA on the slots overlap
+  if (tiles <= num_sms())
+    k_mlp_forward<1><<<grid, InfLayout<1>::threads, InfLayout<1>::smem, (cudaStream_t)stream>>>(dv, n, d_x, d_y);
+  else
+    k_mlp_forward<kSlots><<<grid, InfLayout<kSlots>::threads, InfLayout<kSlots>::smem, (cudaStream_t)stream>>>(dv, n,
+                                                                                                              d_x, d_y);
   MCK(cudaGetLastError());
   return PGFEM_GPU_OK;
 }

@@ -8,12 +8,13 @@
 // increments dt*gamma_dot_a; its prediction only seeds the FP64 Newton.
 //
 // Arithmetic: BF16 operands, FP32 accumulation in tensor memory (TMEM),
-// biases and GELU in FP32.  One CTA of 4 warps owns a tile of 128 points; the
-// tile is the M = 128 dimension of every forward GEMM, each layer is ONE
-// tcgen05.mma chain (K/16 instructions of M128 x N128 x K16) issued by a
-// single thread, completion tracked by tcgen05.commit on an mbarrier, and the
-// epilogue reads the accumulator rows back with tcgen05.ld (warp w owns TMEM
-// lanes 32w..32w+31 = tile rows).
+// biases and GELU in FP32.  A tile of 128 points is the M = 128 dimension of
+// every forward GEMM, each layer is ONE tcgen05.mma chain (K/16 instructions
+// of M128 x N128 x K16) issued by a single thread, completion tracked by
+// tcgen05.commit on an mbarrier, and the epilogue reads the accumulator back
+// with tcgen05.ld: warp w the TMEM lanes (tile rows) of quarter w & 3, and of
+// the columns one half in inference (eight warps a tile, one or three tiles a
+// CTA), one quarter in training (sixteen warps, one tile a CTA).
 //
 // Shared-memory operand layout: every matrix (weights, activations, error
 // terms) is stored as 8x8 BF16 core matrices (128 contiguous bytes, rows of
@@ -33,7 +34,7 @@
 namespace pgb {
 namespace mlp {
 
-constexpr int kIn = 34, kInP = 48, kH = 128, kOut = 12, kOutP = 16, kTile = 128, kThreads = 128;
+constexpr int kIn = 34, kInP = 48, kH = 128, kOut = 12, kOutP = 16, kTile = 128;
 // FP32 master parameter vector: W1[128][34] b1 W2[128][128] b2 W3 b3 W4[12][128] b4
 constexpr int oW1 = 0, ob1 = oW1 + kH * kIn, oW2 = ob1 + kH, ob2 = oW2 + kH * kH, oW3 = ob2 + kH,
               ob3 = oW3 + kH * kH, oW4 = ob3 + kH, ob4 = oW4 + kOut * kH, kNParam = ob4 + kOut;
@@ -48,13 +49,18 @@ constexpr int kScale = 80;
 // shared-memory byte offsets (all multiples of 128)
 constexpr uint32_t sW1 = 0, sW2 = sW1 + kH * kInP * 2, sW3 = sW2 + kH * kH * 2, sW4 = sW3 + kH * kH * 2,
                    sX0 = sW4 + kOutP * kH * 2, sH1 = sX0 + kTile * kInP * 2;
-// inference: kSlots tiles in flight per CTA, eight warps each (a TMEM lane quarter
+// inference: NS tiles (slots) in flight per CTA, eight warps each (a TMEM lane quarter
 // and half of the columns a warp); per slot a feature buffer and one activation
 // buffer reused layer to layer
-constexpr int kSlots = 3, kSlotThreads = 256, kInfThreads = kSlots * kSlotThreads;
-constexpr uint32_t kSlotBytes = (sH1 - sX0) + kTile * kH * 2, sInfBias = sX0 + kSlots * kSlotBytes,
-                   sInfScale = sInfBias + kNPB * 4, sInfMisc = sInfScale + kScale * 4, kInfSmem = sInfMisc + 128;
-static_assert(kInfSmem <= 232448, "inference slots exceed the 227 KB shared-memory limit");
+constexpr int kSlots = 3, kSlotThreads = 256;
+constexpr uint32_t kSlotBytes = (sH1 - sX0) + kTile * kH * 2;
+template <int NS>
+struct InfLayout {
+  static constexpr int threads = NS * kSlotThreads, tmem = NS == 1 ? 128 : 512;
+  static constexpr uint32_t bias = sX0 + NS * kSlotBytes, scale = bias + kNPB * 4, misc = scale + kScale * 4,
+                            smem = misc + 128;
+};
+static_assert(InfLayout<kSlots>::smem <= 232448, "inference slots exceed the 227 KB shared-memory limit");
 // training: H1, H2, H3 kept for the weight gradients, one error-term buffer
 constexpr uint32_t sH2 = sH1 + kTile * kH * 2, sH3 = sH2 + kTile * kH * 2, sDZ = sH3 + kTile * kH * 2,
                    sTrBias = sDZ + kTile * kH * 2, sTrScale = sTrBias + kNPB * 4,
@@ -232,7 +238,7 @@ __device__ __forceinline__ void load_params(unsigned char *sm, const MlpDev &m, 
 
 // ------------------------------------------------------------- inference --
 // Persistent over tiles of 128 points: y[n][12] = network(x[n][34]) in raw units.
-// Three tiles are in flight per CTA (eight warps, 128 TMEM columns, an mbarrier and
+// NS = 3 tiles are in flight per CTA (eight warps, 128 TMEM columns, an mbarrier and
 // a named barrier each) over one copy of the weights, so that one tile's chain
 // and loads run under the others' epilogues; a slot's next features are loaded
 // into registers beside its layers.  Bound by the GELU epilogues: erff and the
@@ -240,22 +246,25 @@ __device__ __forceinline__ void load_params(unsigned char *sm, const MlpDev &m, 
 // 663,552 points.  Measured there: one tile of four warps a CTA 480 us, three slots of
 // four warps 354, of eight 305 (chunks of 16 columns; of 32 the registers spill,
 // 339).  A shorter erf (0.26 ms) changes BF16 roundings of the activations and with
-// them the output by 1e-4, so erff stays.
+// them the output by 1e-4, so erff stays.  NS = 1 is for calls of at most one tile
+// a CTA: the same arithmetic, less to set up.
 __device__ __forceinline__ void slot_sync(int slot) {
   asm volatile("bar.sync %0, %1;" ::"r"(slot + 1), "n"(kSlotThreads) : "memory");
 }
 
-__global__ void __launch_bounds__(kInfThreads, 1)
+template <int NS>
+__global__ void __launch_bounds__(InfLayout<NS>::threads, 1)
     k_mlp_forward(const MlpDev m, long n, const float *__restrict__ x, float *__restrict__ y) {
+  using L = InfLayout<NS>;
   extern __shared__ __align__(128) unsigned char sm[];
-  float *sb = reinterpret_cast<float *>(sm + sInfBias);
-  float *ss = reinterpret_cast<float *>(sm + sInfScale);
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + sInfMisc + 64);
+  float *sb = reinterpret_cast<float *>(sm + L::bias);
+  float *ss = reinterpret_cast<float *>(sm + L::scale);
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + L::misc + 64);
   const int tid = threadIdx.x, warp = tid >> 5, slot = warp >> 3, st = tid & (kSlotThreads - 1);
   const int half = (warp >> 2) & 1, lrow = st & (kTile - 1);  // columns 64 half .. 64 half + 63 of tile row lrow
-  const uint32_t ab = smem_u32(sm), mb = ab + sInfMisc + 8u * (uint32_t)slot;
-  int *sfail = reinterpret_cast<int *>(sm + sInfMisc + 32) + slot;
-  if (warp == 0) tmem_alloc(smem_u32(tslot), 512);
+  const uint32_t ab = smem_u32(sm), mb = ab + L::misc + 8u * (uint32_t)slot;
+  int *sfail = reinterpret_cast<int *>(sm + L::misc + 32) + slot;
+  if (warp == 0) tmem_alloc(smem_u32(tslot), L::tmem);
   if (st == 0) {
     mbar_init(mb, 1);
     *sfail = 0;
@@ -269,7 +278,7 @@ __global__ void __launch_bounds__(kInfThreads, 1)
   tc_after();
   const uint32_t tbase = *tslot + 128u * (uint32_t)slot;
   const uint32_t tme = tbase + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's lane quarter, column 0
-  const long ntiles = (n + kTile - 1) / kTile, step = (long)gridDim.x * kSlots;
+  const long ntiles = (n + kTile - 1) / kTile, step = (long)gridDim.x * NS;
   const bool x8 = (reinterpret_cast<uintptr_t>(x) & 7) == 0, y16 = (reinterpret_cast<uintptr_t>(y) & 15) == 0;
   uint32_t phase = 0;
   bool fail = false;
@@ -374,7 +383,7 @@ __global__ void __launch_bounds__(kInfThreads, 1)
   tc_before();
   __syncthreads();
   tc_after();
-  if (warp == 0) tmem_free(*tslot, 512);
+  if (warp == 0) tmem_free(*tslot, L::tmem);
 }
 
 // -------------------------------------------------------------- training --

@@ -38,3 +38,17 @@ def test_gradient_copies(gpu, n):
     for name, _ in MO.SHAPES:
         assert rel(a[name], b[name]) <= 2e-3, name
     assert np.array_equal(m.loss_grad(x, t)[1], g)
+
+
+# one tile more than there are CTAs takes the kernel with three tiles in flight
+@pytest.mark.parametrize("n", [1, 128, 129, 128 * 148 - 127, 128 * 148, 128 * 148 + 1])
+def test_predict_of_few_rows_equals_that_of_many(gpu, n):
+    import torch
+    many = 128 * 500
+    m, _, x, _, _, _, _ = setup_model(many, seed=3)
+    dx = torch.from_numpy(x).cuda()
+    y, ym = torch.full((n, 12), 7.0, device="cuda"), torch.empty(many, 12, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    m.predict_device(many, dx.data_ptr(), ym.data_ptr(), st)
+    m.predict_device(n, dx.data_ptr(), y.data_ptr(), st)
+    assert torch.equal(y, ym[:n])
