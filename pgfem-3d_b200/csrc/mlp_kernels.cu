@@ -66,8 +66,9 @@ int check_dev() {
     cudaGetLastError();
     return PGFEM_GPU_ENODEV;
   }
-  cudaDeviceProp p;
-  if (cudaGetDeviceProperties(&p, dev) != cudaSuccess || p.major != 10) return PGFEM_GPU_ENODEV;
+  int major = 0;  // the whole property structure takes 2 ms to fill
+  if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess || major != 10)
+    return PGFEM_GPU_ENODEV;
   return PGFEM_GPU_OK;
 }
 
@@ -167,6 +168,11 @@ int pgfem_mlp_create(unsigned long long seed, pgfem_mlp **out) {
     cudaGetLastError();
     return fail(PGFEM_GPU_ENOMEM);
   }
+  // the gradient copies of the largest batch (23 MB at 148 SMs) with the other buffers, as
+  // the first training call took 0.2 to 0.4 ms to allocate them; a device without room for
+  // them still predicts, and trains on the copies its batches need
+  grow(&m->part, &m->part_n, (long)num_sms() * kNParam);
+  if (m->part && cudaMemset(m->part, 0, sizeof(float) * m->part_n)) return fail(PGFEM_GPU_ECUDA);
   if (cudaMemset(m->grad, 0, sizeof(float) * kNParam) || cudaMemset(m->mom, 0, sizeof(float) * kNParam) ||
       cudaMemset(m->vel, 0, sizeof(float) * kNParam) || cudaMemset(m->w, 0, sizeof(__nv_bfloat16) * kNPW) ||
       cudaMemset(m->bias, 0, sizeof(float) * kNPB) || cudaMemset(m->err, 0, sizeof(unsigned)) ||

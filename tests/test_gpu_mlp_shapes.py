@@ -52,3 +52,17 @@ def test_predict_of_few_rows_equals_that_of_many(gpu, n):
     m.predict_device(many, dx.data_ptr(), ym.data_ptr(), st)
     m.predict_device(n, dx.data_ptr(), y.data_ptr(), st)
     assert torch.equal(y, ym[:n])
+
+
+def test_first_training_call_allocates_no_gradient_copies(gpu):
+    import torch
+    n = 20000
+    nets = [setup_model(n, seed=4) for _ in range(2)]
+    x, t = (torch.from_numpy(nets[0][k].astype(np.float32)).cuda() for k in (2, 3))
+    used = []
+    for net in nets:  # the first call of the process may load code
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        net[0].train_device(n, x.data_ptr(), t.data_ptr(), epochs=1, batch=8192)
+        used.append(free - torch.cuda.mem_get_info()[0])
+    assert used[1] <= 2 << 20  # the row order and the losses; the copies of 64 tiles take 10 MB
