@@ -1088,19 +1088,16 @@ int build_gather(pgfem_gpu_ctx *c, const std::vector<int> &dof, const std::vecto
     for (int i = 2; mask[n] && i >= 0; i--)
       if (dof[(size_t)i * nn + n] > 0) grp[n] = gid[owner[dof[(size_t)i * nn + n] - 1]];
   std::vector<int> off((size_t)ng + 1), two((size_t)3 * ng), so((size_t)ng + 1), eo((size_t)ng + 1);
-  int *d_grp = nullptr, *d_two = nullptr, *d_err = nullptr, *d_off = nullptr;
-  int4 *d_row = nullptr;
+  int4 *d_row = nullptr;  // scratch of the construction, in one piece
+  if (cudaMalloc(&d_row, sizeof(int4) * ng + sizeof(int) * (3 * ng + (ng + 1) + 1 + nn))) {
+    cudaGetLastError();
+    return PGFEM_GPU_ENOMEM;
+  }
+  int *d_two = reinterpret_cast<int *>(d_row + ng), *d_off = d_two + 3 * ng, *d_err = d_off + ng + 1, *d_grp = d_err + 1;
   auto done = [&](int r) {
-    for (void *p : {(void *)d_grp, (void *)d_two, (void *)d_err, (void *)d_off, (void *)d_row})
-      if (p) cudaFree(p);
+    cudaFree(d_row);
     return r;
   };
-  if (cudaMalloc(&d_grp, sizeof(int) * nn) || cudaMalloc(&d_two, sizeof(int) * 3 * ng) ||
-      cudaMalloc(&d_err, sizeof(int)) || cudaMalloc(&d_off, sizeof(int) * 2 * (ng + 1)) ||
-      cudaMalloc(&d_row, sizeof(int4) * ng)) {
-    cudaGetLastError();
-    return done(PGFEM_GPU_ENOMEM);
-  }
   const unsigned b4 = (unsigned)((4 * ne + 255) / 256), bg = (unsigned)((ng + 127) / 128);
   cudaStream_t s = c->stream;
   auto bad = [](cudaError_t e) { return e != cudaSuccess; };
@@ -1171,6 +1168,21 @@ int build_gather(pgfem_gpu_ctx *c, const std::vector<int> &dof, const std::vecto
   c->gl = gl;
   c->gather = true;
   return done(PGFEM_GPU_OK);
+}
+
+// build_gather for a context that does without the lists when they cannot be built
+// or find no room: the scatter needs neither them nor the records.
+int build_gather_if(pgfem_gpu_ctx *c, const std::vector<int> &dof, const std::vector<int> &rowptr0,
+                    const std::vector<int> &rowlen, const std::vector<uint8_t> &mask) {
+  const long bytes = c->bytes;
+  const int r = build_gather(c, dof, rowptr0, rowlen, mask);
+  if (c->gather) return r;
+  for (void *&p : c->g_mem) {
+    if (p) cudaFree(p);
+    p = nullptr;
+  }
+  c->bytes = bytes;
+  return r == PGFEM_GPU_ENOMEM ? PGFEM_GPU_OK : r;
 }
 
 // Greedy colouring: elements of one colour share no node, so their R and K
@@ -1425,8 +1437,6 @@ int pgfem_gpu_create(const pgfem_mesh_desc *m, const pgfem_material_desc *mat, c
     if (ce != cudaSuccess) return fail(PGFEM_GPU_ECUDA);
     if (herr) return fail(PGFEM_GPU_EPATTERN);
   }
-  // linear tets: lists of the row owners
-  if (m->nne == 4 && c->mat.dev_pot != 2 && (r = build_gather(c, dof, rowptr0, rowlen, mask))) return fail(r);
   // quadratic-tet path: processing order, scatter blocks in that
   // order, the second stream that zeroes K
   if (m->nne == 10 && c->model != PGFEM_MODEL_CP && c->mat.dev_pot != 2) {
@@ -1446,14 +1456,12 @@ int pgfem_gpu_create(const pgfem_mesh_desc *m, const pgfem_material_desc *mat, c
   // crystal plasticity buffers (rotations SoA, F, point outputs)
   if (c->model == PGFEM_MODEL_CP) {
     std::vector<double> Rs((size_t)9 * ne);
-    c->cp_rot = cp_rotations_orthogonal(m->R_cp, ne);
     for (long e = 0; e < ne; e++)
       for (int i = 0; i < 9; i++) Rs[(size_t)i * ne + e] = m->R_cp[e * 9 + i];
     if ((r = upload(c, &c->cp_R, Rs.data(), Rs.size())) || (r = dalloc(c, &c->cp_F, (size_t)9 * ne)) ||
         (r = dalloc(c, &c->cp_detJw, ne)) || (r = dalloc(c, &c->cp_out, (size_t)kCpOut * c->nqp)) ||
         (r = dalloc(c, &c->cp_iters, c->nqp)) || (r = dalloc(c, &c->cp_counter, 1)) ||
-        (r = dalloc(c, &c->cp_fallbacks, 1)) || (r = dalloc(c, &c->cp_conv, c->nqp)) ||
-        (c->cp_rot && (r = dalloc(c, &c->cp_rec, (size_t)kCxRec * ne))))
+        (r = dalloc(c, &c->cp_fallbacks, 1)) || (r = dalloc(c, &c->cp_conv, c->nqp)))
       return fail(r);
     std::vector<double> Fn((size_t)9 * c->nqp, 0.0);  // F at t_n: identity until the first commit
     for (long q = 0; q < c->nqp; q++) Fn[0 * c->nqp + q] = Fn[4 * c->nqp + q] = Fn[8 * c->nqp + q] = 1.0;
@@ -1475,6 +1483,13 @@ int pgfem_gpu_create(const pgfem_mesh_desc *m, const pgfem_material_desc *mat, c
       cudaMemcpyAsync(c->state_nm1, s0.data(), s0.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream);
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) return fail(PGFEM_GPU_ECUDA);
   }
+  // last, as the context does without them: the crystal-frame kernels' records and, for
+  // linear tets, the lists of the row owners
+  if (c->model == PGFEM_MODEL_CP)
+    c->cp_rot = cp_rotations_orthogonal(m->R_cp, ne) && !dalloc(c, &c->cp_rec, (size_t)kCxRec * ne);
+  if (m->nne == 4 && c->mat.dev_pot != 2 && (c->model != PGFEM_MODEL_CP || c->cp_rot) &&
+      (r = build_gather_if(c, dof, rowptr0, rowlen, mask)))
+    return fail(r);
   *out = c;
   return PGFEM_GPU_OK;
 }
