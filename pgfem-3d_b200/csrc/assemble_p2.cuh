@@ -260,8 +260,8 @@ constexpr int kP2Run = 8;
 //   [64, 114)  node-pair positions pos[a][b] (uint16, column offset of b's block in a's rows)
 //   [114, 117) free-component masks of the ten nodes (bytes)
 //   [117, 119) 4 bits per node: its local number in the previous element of the
-//              processing order, 15 when not there
-//   [119]      bit a: node a is in the next element too
+//              processing order, 15 when not there (or when either holds it twice)
+//   [119]      bit a: node a is in the next element too (once in both)
 constexpr int kEBW = 120;
 constexpr int kEBRes = 32, kEBPos = 64, kEBMask = 114, kEBPrev = 117, kEBNext = 119;
 // the four-point rule: point q has barycentric coordinate A at corner (q + 1) mod 4, B at the others
@@ -308,16 +308,29 @@ __global__ void k_build_eblock(const int *conn, long ne, const int *dof, long nn
   const long ep = es > 0 ? (perm ? (long)perm[es - 1] : es - 1) : -1;
   const long en = es + 1 < ne ? (perm ? (long)perm[es + 1] : es + 1) : -1;
   unsigned long long prev = 0;
-  int next = 0;
+  int next = 0, ne_[10], np_[10], nn_[10];
   for (int a = 0; a < 10; a++) {
-    const int n = conn[(long)a * ne + e];
+    ne_[a] = conn[(long)a * ne + e];
+    np_[a] = ep >= 0 ? conn[(long)a * ne + ep] : -1;
+    nn_[a] = en >= 0 ? conn[(long)a * ne + en] : -1;
+  }
+  for (int a = 0; a < 10; a++) {
+    const int n = ne_[a];
     const unsigned mk = mask[n];
+    // handed on only when the node stands once in either element (a mid-side node may
+    // coincide with its corner): an entry then has one place in both
+    int own = 0, inp = 0, inn = 0;
     unsigned long long pa = 15;
     for (int x = 0; x < 10; x++) {
-      if (ep >= 0 && conn[(long)x * ne + ep] == n) pa = x;
-      if (en >= 0 && conn[(long)x * ne + en] == n) next |= 1 << a;
+      own += ne_[x] == n;
+      inn += nn_[x] == n;
+      if (np_[x] == n) {
+        inp++;
+        pa = x;
+      }
     }
-    prev |= pa << (4 * a);
+    prev |= (own == 1 && inp == 1 ? pa : 15ull) << (4 * a);
+    next |= (own == 1 && inn == 1 ? 1 : 0) << a;
     for (int i = 0; i < 3; i++) {
       const bool fr = (mk >> i) & 1u;
       o[a * 3 + i] = fr ? rowptr0[n] + __popc(mk & ((1u << i) - 1u)) * rowlen[n] : -1;
