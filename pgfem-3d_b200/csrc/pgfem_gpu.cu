@@ -1026,6 +1026,8 @@ int assemble_device(pgfem_gpu_ctx *c, const double *d_u, const double *d_presc, 
 int read_status(pgfem_gpu_ctx *c, pgfem_gpu_status *st, bool clear) {
   unsigned long long h[4];
   CK(cudaMemcpyAsync(h, c->status, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+  // cleared before this returns: the caller's next kernels count on other streams
+  if (clear) CK(cudaMemsetAsync(c->status, 0, sizeof(h), c->stream));
   CK(cudaStreamSynchronize(c->stream));
   if (st) {
     st->inverted = (long)h[0];
@@ -1033,7 +1035,6 @@ int read_status(pgfem_gpu_ctx *c, pgfem_gpu_status *st, bool clear) {
     st->bad_diagonal = (long)h[2];
     st->other = (long)h[3];
   }
-  if (clear) CK(cudaMemsetAsync(c->status, 0, sizeof(h), c->stream));
   return PGFEM_GPU_OK;
 }
 
