@@ -122,6 +122,8 @@ int pgfem_mesh_box_tet(int n, int nne, int periodic, long *nn, long *ne, double 
 int pgfem_gpu_create(const pgfem_mesh_desc *mesh, const pgfem_material_desc *mat, const int *Ap,
                      const int *Ai, long nrows, pgfem_gpu_ctx **ctx);
 int pgfem_gpu_destroy(pgfem_gpu_ctx *ctx);
+/* The first change to colour mode builds the element colours (synchronises; some
+ * 0.1 s per million elements; ENOMEM leaves the mode as it was). */
 int pgfem_gpu_set_scatter_mode(pgfem_gpu_ctx *ctx, int mode);
 /* Tests of the failure path (no counterpart in the reference): the bound of
  * the producer/consumer hand-off waits of the linear-tet R+K kernel (seconds,

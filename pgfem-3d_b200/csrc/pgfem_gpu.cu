@@ -17,6 +17,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <vector>
 
 #include "assemble.cuh"
@@ -1506,13 +1507,28 @@ int pgfem_gpu_destroy(pgfem_gpu_ctx *c) {
 int pgfem_gpu_set_scatter_mode(pgfem_gpu_ctx *c, int mode) {
   if (!c || (mode != PGFEM_SCATTER_ATOMIC && mode != PGFEM_SCATTER_COLOUR)) return PGFEM_GPU_EINVAL;
   if (mode == PGFEM_SCATTER_COLOUR && !c->colour_elems) {  // the colours, on first use
-    std::vector<int> conn((size_t)c->nne * c->ne), dof((size_t)3 * c->nn), el;
-    CK(cudaMemcpyAsync(conn.data(), c->conn, sizeof(int) * conn.size(), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(dof.data(), c->dof, sizeof(int) * dof.size(), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    build_colours(c, conn, dof, el, c->colour_off);
-    if (int r = upload(c, &c->colour_elems, el.data(), el.size())) return r;
-    CK(cudaStreamSynchronize(c->stream));
+    const long bytes = c->bytes;
+    int *elems = nullptr, r;
+    try {
+      std::vector<int> conn((size_t)c->nne * c->ne), dof((size_t)3 * c->nn), el;
+      std::vector<long> off;
+      CK(cudaMemcpyAsync(conn.data(), c->conn, sizeof(int) * conn.size(), cudaMemcpyDeviceToHost, c->stream));
+      CK(cudaMemcpyAsync(dof.data(), c->dof, sizeof(int) * dof.size(), cudaMemcpyDeviceToHost, c->stream));
+      CK(cudaStreamSynchronize(c->stream));
+      build_colours(c, conn, dof, el, off);
+      r = upload(c, &elems, el.data(), el.size());
+      if (!r && cudaStreamSynchronize(c->stream) != cudaSuccess) r = PGFEM_GPU_ECUDA;
+      if (!r) c->colour_off.swap(off);
+    } catch (const std::bad_alloc &) {
+      r = PGFEM_GPU_ENOMEM;
+    }
+    if (r) {
+      cudaGetLastError();
+      if (elems) cudaFree(elems);
+      c->bytes = bytes;
+      return r;
+    }
+    c->colour_elems = elems;
   }
   c->scatter_mode = mode;
   return PGFEM_GPU_OK;
